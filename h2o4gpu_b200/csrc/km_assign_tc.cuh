@@ -53,20 +53,34 @@ namespace tc {
 
 constexpr int kBM = 128;
 constexpr int kThreads = 768;  // producer, 2 MMA issuers, spare, 2 x 4 converter warps, 3 x 4 epilogue warps
-constexpr int kStages = 5;
 constexpr int kAcc = 3;        // TMEM accumulators
 constexpr int kMaxD = 64;
 constexpr int kMaxNPad = 128;
 constexpr int kTmemCols = 512;
 
-enum Bar { FULL = 0, EMPTY = kStages, A_READY = 2 * kStages, A_EMPTY = 2 * kStages + 2,
-           ACC_FULL = 2 * kStages + 4, ACC_EMPTY = 2 * kStages + 4 + kAcc, B_FULL = 2 * kStages + 4 + 2 * kAcc,
-           NUM_BARS = 2 * kStages + 5 + 2 * kAcc };
+// Row tiles in flight: five of raw float32 rows (32 KB each at d = 64), ten of fp16 upper halves (16 KB each).
+// Ten is even on purpose: a stage then always serves the same MMA issuer.
+constexpr int stages_of(bool pre) { return pre ? 10 : 5; }
+template <bool PRE>
+struct Bars {
+  static constexpr int NS = stages_of(PRE);
+  static constexpr int FULL = 0, EMPTY = NS, A_READY = 2 * NS, A_EMPTY = 2 * NS + 2, ACC_FULL = 2 * NS + 4,
+                       ACC_EMPTY = 2 * NS + 4 + kAcc, B_FULL = 2 * NS + 4 + 2 * kAcc, COUNT = 2 * NS + 5 + 2 * kAcc;
+};
 
 // shared memory: [bh panel][bl panel][stages][cn][barriers][misc]; d is 32 or 64
-inline size_t smem_bytes(int d, int npad) {
-  size_t P = d / 32;
-  return 1024 + 2 * (size_t)npad * 128 + (size_t)kStages * P * 16384 + (size_t)npad * 4 + NUM_BARS * 8 + 64;
+inline size_t smem_bytes(int d, int npad, bool pre) {
+  const size_t stage = pre ? 16384 : (size_t)(d / 32) * 16384;
+  const size_t bars = pre ? Bars<true>::COUNT : Bars<false>::COUNT;
+  return 1024 + 2 * (size_t)npad * 128 + (size_t)stages_of(pre) * stage + (size_t)npad * 4 + bars * 8 + 64;
+}
+// Rows a CTA can list for the exact pass: every CTA has a segment of its own in the list, so that appending
+// needs no global counter (at a few per cent of the rows the same-address atomics would take longer than the
+// distances).
+inline size_t amb_seg_rows(size_t rows, int num_sms) {
+  const size_t tiles = (rows + kBM - 1) / kBM;
+  const size_t grid = std::min<size_t>(std::max<size_t>(tiles, 1), (size_t)num_sms);
+  return (tiles + grid - 1) / grid * kBM;
 }
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -258,6 +272,21 @@ __device__ __forceinline__ float split_tolerance(float tol_rel, float tol_floor,
   return tol_rel * (xn + cn_max) * sxsb + tol_floor * (sx * sqrtf(xn) + sb2 * sqrtf(cn_max));
 }
 
+// The same when the row enters the product rounded to its upper half only (two terms, xh.bh + xh.bl): the
+// dropped part is ey.b_j with ey = y - xh, whose length `ey` is known exactly.  Only its difference between two
+// centroids matters, |ey.(b_j - b_best)| <= ey * 2 sb |c_j - c_best|; and for the true nearest centroid j,
+// |x - c_j| <= |x - c_best| = dist, so |c_j - c_best| <= 2 dist.  dist^2 = |x|^2 + score, with the score's own
+// error (at most ey * 2 sb max|c| on top of the three-term bound) added.  The bound shrinks with the distance of a
+// row to its centre, which is what keeps the exact pass short: two centroids in one cluster are close to
+// each other, so rounding the row moves their scores together.
+__device__ __forceinline__ float split_tolerance_upper(float tol_rel, float tol_floor, float xn, float ey, float best,
+                                                       float cn_max, float sx, float sxsb) {
+  const float t3 = split_tolerance(tol_rel, tol_floor, xn, cn_max, sx, sxsb);
+  const float sb2 = 2.0f * sxsb / sx;
+  const float dist_sq = xn + (best + t3 + ey * sb2 * sqrtf(cn_max)) / sxsb;
+  return t3 + 1.001f * (2.0f * ey * sb2 * sqrtf(fmaxf(dist_sq, 0.f)));
+}
+
 // |x|^2 of every row (float), once per upload: the error bound of a row's scores.  The
 // tensor-core paths have d % 4 == 0 and 16-byte aligned rows: a row is shared by lpr lanes
 // loading a float4 each, four sets of rows per loop trip.
@@ -328,41 +357,63 @@ prep_kernel(const float* __restrict__ C, const float* __restrict__ cnorm, int k,
   }
 }
 
-// The rows of X split once into the two fp16 operands of the product (the arithmetic of the
-// converter warps below: y = x * sx, upper half = fp16(y), lower half = fp16(y - upper)), so that
-// the E-step can read them with TMA straight into the layout the MMA consumes and needs no
-// conversion per iteration.  Same bytes per element as the float32 matrix (2 + 2).
+// The rows of X rounded once to fp16 (y = x * sx, upper half = fp16(y)), so that the E-step reads two bytes per
+// element instead of four, straight into the layout the MMA consumes, with no conversion per iteration; and per
+// row |x|^2 and |y - fp16(y)|, the two numbers the error bound of a score needs (split_tolerance_upper).
+// 64 columns: sixteen lanes share a row, one float4 each, eight rows per lane in flight.  Bound by HBM: reads
+// 256 and writes 136 bytes per row; 1e7 rows in MEASURED_SPLIT.
 __global__ void __launch_bounds__(256)
-split_rows_kernel(const float* __restrict__ X, size_t count, float sx, __half* __restrict__ xh,
-                  __half* __restrict__ xl) {
-  const size_t nvec = count / 8;
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < nvec; i += (size_t)gridDim.x * blockDim.x) {
-    const float4 a = __ldcs(reinterpret_cast<const float4*>(X) + 2 * i);
-    const float4 b = __ldcs(reinterpret_cast<const float4*>(X) + 2 * i + 1);
-    const float y[8] = {a.x * sx, a.y * sx, a.z * sx, a.w * sx, b.x * sx, b.y * sx, b.z * sx, b.w * sx};
-    uint32_t hi[4], lo[4];
+split_rows_kernel(const float* __restrict__ X, size_t n, float sx, __half* __restrict__ xh, float2* __restrict__ rowq) {
+  constexpr int U = 8;
+  const int lane = threadIdx.x & 31;
+  const int g = lane >> 4, l = lane & 15;
+  const size_t warp = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const size_t nwarp = ((size_t)gridDim.x * blockDim.x) >> 5;
+  for (size_t base = warp * 2 * U; base < n; base += nwarp * 2 * U) {
+    float4 v[U];
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      const __half2 h = __floats2half2_rn(y[2 * c], y[2 * c + 1]);
-      const float2 f = __half22float2(h);
-      const __half2 l = __floats2half2_rn(y[2 * c] - f.x, y[2 * c + 1] - f.y);
-      hi[c] = *reinterpret_cast<const uint32_t*>(&h);
-      lo[c] = *reinterpret_cast<const uint32_t*>(&l);
+    for (int u = 0; u < U; ++u) {
+      const size_t row = base + 2 * u + g;
+      v[u] = (row < n) ? __ldcs(reinterpret_cast<const float4*>(X + row * 64) + l) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
-    reinterpret_cast<uint4*>(xh)[i] = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-    reinterpret_cast<uint4*>(xl)[i] = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const size_t row = base + 2 * u + g;
+      const float y0 = v[u].x * sx, y1 = v[u].y * sx, y2 = v[u].z * sx, y3 = v[u].w * sx;
+      const __half2 h01 = __floats2half2_rn(y0, y1), h23 = __floats2half2_rn(y2, y3);
+      const float2 f01 = __half22float2(h01), f23 = __half22float2(h23);
+      const float e0 = y0 - f01.x, e1 = y1 - f01.y, e2 = y2 - f23.x, e3 = y3 - f23.y;   // exact
+      float q = fmaf(v[u].x, v[u].x, fmaf(v[u].y, v[u].y, fmaf(v[u].z, v[u].z, v[u].w * v[u].w)));
+      float e = fmaf(e0, e0, fmaf(e1, e1, fmaf(e2, e2, e3 * e3)));
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) {
+        q += __shfl_xor_sync(0xffffffffu, q, o);
+        e += __shfl_xor_sync(0xffffffffu, e, o);
+      }
+      if (row < n) {
+        *reinterpret_cast<uint2*>(xh + row * 64 + l * 4) =
+            make_uint2(*reinterpret_cast<const uint32_t*>(&h01), *reinterpret_cast<const uint32_t*>(&h23));
+        if (l == 0) rowq[row] = make_float2(q, sqrtf(e));
+      }
+    }
   }
 }
 
 template <int D, bool PRE>
 __global__ void __launch_bounds__(kThreads, 1)
-assign_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmXl,
-                 const __grid_constant__ CUtensorMap tmBhi,
+assign_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmBhi,
                  const __grid_constant__ CUtensorMap tmBlo, const float* __restrict__ cn_pad,
-                 const float* __restrict__ xnorm, int* __restrict__ labels, size_t n, int n_tiles, int npad,
-                 IterState* st, int count_changes, unsigned int* __restrict__ amb_rows, float tol_rel, float tol_floor,
+                 const float* __restrict__ xnorm, const float2* __restrict__ rowq, int* __restrict__ labels, size_t n,
+                 int n_tiles, int npad, IterState* st, int count_changes, unsigned int* __restrict__ amb_rows,
+                 unsigned int* __restrict__ amb_seg, unsigned int amb_seg_cap, float tol_rel, float tol_floor,
                  float sx, float sxsb, unsigned int* __restrict__ moved_bits, uint4* __restrict__ amb_near,
-                 unsigned int wait_iters) {
+                 int gate, unsigned int wait_iters) {
+  // both variants are queued when a split copy exists; the device decides which one works (see IterState)
+  if (gate && (st->full_rows != 0) == PRE) return;
+  using B = Bars<PRE>;
+  constexpr int kStages = B::NS;
+  constexpr int FULL = B::FULL, EMPTY = B::EMPTY, A_READY = B::A_READY, A_EMPTY = B::A_EMPTY, ACC_FULL = B::ACC_FULL,
+                ACC_EMPTY = B::ACC_EMPTY, B_FULL = B::B_FULL, NUM_BARS = B::COUNT;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw_u32 = smem_u32(smem_raw);
   const uint32_t base = (raw_u32 + 1023u) & ~1023u;
@@ -373,7 +424,7 @@ assign_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
   const uint32_t b_panel = (uint32_t)npad * 128u;       // one fp16 panel: npad rows x 64 halves
   const uint32_t off_blo = b_panel;
   const uint32_t off_stage = 2u * b_panel;
-  constexpr uint32_t stage_bytes = (uint32_t)P * 16384u;
+  constexpr uint32_t stage_bytes = PRE ? 16384u : (uint32_t)P * 16384u;
   const uint32_t off_cn = off_stage + kStages * stage_bytes;
   const uint32_t off_bar = (off_cn + (uint32_t)npad * 4u + 7u) & ~7u;
   const uint32_t off_misc = off_bar + NUM_BARS * 8;
@@ -381,6 +432,7 @@ assign_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
   volatile uint32_t* tmem_holder = reinterpret_cast<volatile uint32_t*>(sm + off_misc);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(sm + off_misc + 4);
   volatile int* issued_upto = reinterpret_cast<volatile int*>(sm + off_misc + 8);  // [2]: last tile counter issued by each issuer
+  unsigned int* amb_n = reinterpret_cast<unsigned int*>(sm + off_misc + 20);       // rows this CTA has listed
   auto bar = [&](int i) { return base + off_bar + (uint32_t)i * 8u; };
 
   const int tid = threadIdx.x;
@@ -396,6 +448,7 @@ assign_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
     abort_flag[3] = (int)wait_iters;
     issued_upto[0] = -1;
     issued_upto[1] = -1;
+    *amb_n = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   for (int i = tid; i < npad; i += kThreads) cn_s[i] = cn_pad[i];
@@ -431,10 +484,8 @@ assign_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
         if (!ok) break;
         mbar_expect_tx(bar(FULL + s), stage_bytes);
         if (PRE) {
-          // the row tile arrives split already: upper halves, then lower halves, each 128 rows x 64 halves in
-          // the layout the MMA reads
+          // the row tile arrives rounded already: 128 rows x 64 upper halves in the layout the MMA reads
           tma_load_2d(base + off_stage + s * stage_bytes, &tmX, 0, tile * kBM, bar(FULL + s));
-          tma_load_2d(base + off_stage + s * stage_bytes + 16384u, &tmXl, 0, tile * kBM, bar(FULL + s));
         } else {
 #pragma unroll
           for (int p = 0; p < P; ++p)
@@ -493,13 +544,13 @@ assign_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
         const uint32_t acc = tmem_base + (uint32_t)a * 128u;
 #pragma unroll
         for (int term = 0; term < 3; ++term) {
+          if (PRE && term == 1) continue;   // no lower halves of the rows
 #pragma unroll
           for (int kk = 0; kk < KS; ++kk) {
             const uint32_t a_col = a_hi + (term == 1 ? 32u : 0u) + kk * 8u;
             const uint64_t bd = (term == 2) ? bdesc_lo[kk] : bdesc_hi[kk];
             if (PRE) {
-              const uint32_t a_smem = base + off_stage + (uint32_t)s * stage_bytes + (term == 1 ? 16384u : 0u) + kk * 32u;
-              tc_mma_ss(acc, smem_desc_sw128(a_smem), bd, idesc, 1u);
+              tc_mma_ss(acc, smem_desc_sw128(base + off_stage + (uint32_t)s * stage_bytes + kk * 32u), bd, idesc, 1u);
             } else {
               tc_mma_ts(acc, a_col, bd, idesc, 1u);
             }
@@ -610,9 +661,15 @@ assign_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
       // that their DRAM round trip hides behind the wait and the arithmetic
       const size_t row = (size_t)tile * kBM + row_in_tile;
       int old_label = -1;
-      float xn = 0.f;
+      float xn = 0.f, ey = 0.f;
       if (row < n) {
-        xn = xnorm[row];
+        if (gate) {   // a split copy exists, and |x|^2 beside it
+          const float2 q = __ldcs(rowq + row);
+          xn = q.x;
+          ey = q.y;
+        } else {
+          xn = xnorm[row];
+        }
         if (count_changes) old_label = labels[row];
       }
       ok = mbar_wait(bar(ACC_FULL + a), pha, abort_flag, 7, i);
@@ -642,8 +699,9 @@ assign_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
       }
       const float best = fminf(m0, m1);
       // rows with a second score within the error bound of the split product (scores carry the
-      // factor sx*sb) go to the exact re-evaluation pass; without that pass only exact ties count
-      const float tol = (amb_rows != nullptr) ? split_tolerance(tol_rel, tol_floor, xn, cn_max, sx, sxsb) : 0.f;
+      // factor sx*sb) go to the exact re-evaluation pass
+      const float tol = PRE ? split_tolerance_upper(tol_rel, tol_floor, xn, ey, best, cn_max, sx, sxsb)
+                            : split_tolerance(tol_rel, tol_floor, xn, cn_max, sx, sxsb);
       const float thr = best + tol;
       // pass 2: one bit per column whose score is within the bound of the best
       uint32_t near[kMaxNPad / 32];
@@ -675,8 +733,8 @@ assign_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
       }
       bool moved = false;
       if (row < n) {
-        if (amb_rows != nullptr && n_near != 1) {
-          const unsigned int pos = atomicAdd(&st->amb_count, 1u);
+        if (n_near != 1) {
+          const unsigned int pos = blockIdx.x * amb_seg_cap + atomicAdd(amb_n, 1u);
           amb_rows[pos] = (unsigned int)row;
           amb_near[pos] = make_uint4(near[0], near[1], near[2], near[3]);   // the candidates of the exact pass
         } else {
@@ -700,7 +758,11 @@ assign_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
   }
 
   __syncthreads();
-  if (tid == 0 && *abort_flag) atomicMax(&st->error, *abort_flag);
+  if (tid == 0) {
+    if (*abort_flag) atomicMax(&st->error, *abort_flag);
+    amb_seg[blockIdx.x] = *amb_n;
+    if (*amb_n) atomicAdd(&st->amb_count, *amb_n);
+  }
   if (warp == 1) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)kTmemCols)

@@ -280,7 +280,8 @@ struct IterState {
   int relocated;                // relocations done in the current M-step
   int error;                    // sticky device-side error word (0 = none)
   unsigned int amb_count;       // rows handed to the exact re-evaluation pass in the current E-step
-  unsigned int pad0;
+  unsigned int full_rows;       // 1: an E-step on rounded rows listed too many for the exact pass; the fit goes on with
+                                // the kernel that reads the whole rows (set by close_kernel, cleared when a fit begins)
   double shift_sq;              // summed squared centroid shift of the current M-step
   double inertia;               // scratch for the inertia pass
 };

@@ -105,6 +105,7 @@ struct Shard {
   const T* xpad_of = nullptr;
   size_t xpad_rows = 0;
   size_t amb_cap = 0;
+  unsigned int* amb_seg = nullptr;   // rows each CTA of the small-table kernel has listed in its segment of amb_rows
   uint4* amb_near = nullptr;         // per listed row: bit mask of the candidate centroids (small tables)
   size_t amb_near_cap = 0;
   unsigned int* amb_log = nullptr;
@@ -241,6 +242,27 @@ struct Engine : EngineBase {
   // the sums and everything else keep reading the rows as they are).
   int dtc() const { return (d + 3) / 4 * 4; }
   int ensure_xpad(Shard<T>& s);
+  // list of the rows handed to the exact pass (cut into one segment per CTA for the small-table kernel, which
+  // also leaves a mask of candidates per listed row)
+  int ensure_amb(Shard<T>& s, bool near) {
+    const size_t need = std::max(s.rows, tc::amb_seg_rows(s.rows, s.num_sms) * (size_t)s.num_sms);
+    if (s.amb_cap < need) {
+      km_free(s.amb_rows);
+      s.amb_rows = nullptr;
+      s.amb_cap = 0;
+      KM_CUDA(km_malloc(&s.amb_rows, need * sizeof(unsigned int)));
+      s.amb_cap = need;
+    }
+    if (near && s.amb_near_cap < need) {
+      km_free(s.amb_near);
+      s.amb_near = nullptr;
+      s.amb_near_cap = 0;
+      KM_CUDA(km_malloc(&s.amb_near, need * sizeof(uint4)));
+      s.amb_near_cap = need;
+    }
+    if (near && !s.amb_seg) KM_CUDA(km_malloc(&s.amb_seg, (size_t)s.num_sms * sizeof(unsigned int)));
+    return KM_OK;
+  }
   const T* xtc(const Shard<T>& s) const { return d % 4 == 0 ? s.X : s.xpad; }
   int stream_refresh(Shard<T>& s);   // operand table and plan of the streaming kernel for the current centroids
   int tc_refresh(Shard<T>& s);  // split the current centroids for the tensor-core kernel
@@ -393,7 +415,7 @@ void Engine<T>::destroy() {
     s.tcbp.release();
     s.tcwp.release();
     s.tcsp.release();
-    km_free(s.amb_rows); km_free(s.amb_near); km_free(s.amb_log); km_free(s.xpad);
+    km_free(s.amb_rows); km_free(s.amb_near); km_free(s.amb_seg); km_free(s.amb_log); km_free(s.xpad);
     km_free(s.X_owned); km_free(s.raw); km_free(s.w); km_free(s.labels); km_free(s.dist); km_free(s.gacc);
     km_free(s.pacc); km_free(s.pflush); km_free(s.labels_prev); km_free(s.moved_bits);
     km_free(s.C[0]); km_free(s.C[1]); km_free(s.Cd[0]); km_free(s.Cd[1]); km_free(s.cnorm); km_free(s.shift_k); km_free(s.empties);
@@ -758,18 +780,7 @@ int Engine<T>::preallocate(int k_, int max_iter) {
       KM_CUDA(km_malloc(&s.moved_bits, (s.rows / 32 + 8) * sizeof(unsigned int)));
       s.labels_prev_cap = s.rows;
     }
-    if (std::is_same<T, float>::value && s.amb_cap < s.rows) {
-      km_free(s.amb_rows);
-      s.amb_rows = nullptr;
-      KM_CUDA(km_malloc(&s.amb_rows, s.rows * sizeof(unsigned int)));
-      s.amb_cap = s.rows;
-    }
-    if (std::is_same<T, float>::value && tc::shape_ok(k_, d) && s.amb_near_cap < s.rows) {
-      km_free(s.amb_near);
-      s.amb_near = nullptr;
-      KM_CUDA(km_malloc(&s.amb_near, s.rows * sizeof(uint4)));
-      s.amb_near_cap = s.rows;
-    }
+    if (std::is_same<T, float>::value) KM_TRY(ensure_amb(s, tc::shape_ok(k_, d)));
   }
   (void)max_iter;
   return KM_OK;
@@ -1202,18 +1213,7 @@ int Engine<T>::tc_refresh(Shard<T>& s) {
     if (!tc::pick_scales(xmax, std::max(xmax, cbound), &tc_sx, &tc_sb))
       KM_FAIL(KM_EINVAL, "data magnitude outside the range of the tensor-core kernel");
     if (s.rows > 0xffffffffULL) KM_FAIL(KM_EINVAL, "shard too large for the tensor-core kernel");
-    if (s.amb_cap < s.rows) {
-      km_free(s.amb_rows);
-      s.amb_rows = nullptr;
-      KM_CUDA(km_malloc(&s.amb_rows, s.rows * sizeof(unsigned int)));
-      s.amb_cap = s.rows;
-    }
-    if (tc_kind() == 1 && s.amb_near_cap < s.rows) {
-      km_free(s.amb_near);
-      s.amb_near = nullptr;
-      KM_CUDA(km_malloc(&s.amb_near, s.rows * sizeof(uint4)));
-      s.amb_near_cap = s.rows;
-    }
+    KM_TRY(ensure_amb(s, tc_kind() == 1));
     const int kind = tc_kind();
     if (d % 4 != 0) KM_TRY(ensure_xpad(s));
     if (kind == 3) {
@@ -1312,13 +1312,20 @@ int Engine<T>::launch_assign(Shard<T>& s, bool use_tc, bool count_changes) {
       return KM_OK;
     }
     if (use_tc) {
-      launches += 2;
       unsigned int* bits = (count_changes && s.labels_prev_cap >= s.rows) ? s.moved_bits : nullptr;
-      KM_TRY(tc::launch(s.tcp, s.labels, s.st, count_changes, s.amb_rows, tc::tol_rel_of(d), s.num_sms,
-                        s.stream, bits, s.amb_near, tc_split_build));
+      KM_TRY(tc::launch(s.tcp, s.labels, s.st, count_changes, s.amb_rows, s.amb_seg, tc::tol_rel_of(d), s.num_sms,
+                        s.stream, bits, s.amb_near, tc_split_build, &launches));
       s.moved_bits_valid = bits != nullptr;
-      refine_near_kernel<float><<<s.num_sms * 4, kRefineThreads, 0, s.stream>>>(
-          s.X, d, s.C[cur], k, s.amb_rows, s.amb_near, s.st, s.labels, count_changes ? 1 : 0, bits);
+      const size_t tiles = (s.rows + tc::kBM - 1) / tc::kBM;
+      const int n_seg = (int)std::min<size_t>(tiles, (size_t)s.num_sms);
+      auto refine = [&](auto fn) {
+        fn<<<n_seg * kRefineSplit, kRefineThreads, 0, s.stream>>>(
+            s.X, s.Cd[cur], k, s.amb_rows, s.amb_near, s.amb_seg, (unsigned int)tc::amb_seg_rows(s.rows, s.num_sms), n_seg,
+            s.st, s.labels, count_changes ? 1 : 0, bits);
+      };
+      if (d == 32) refine(refine_near_kernel<32>);
+      else refine(refine_near_kernel<64>);
+      ++launches;
       KM_CUDA(cudaGetLastError());
       return KM_OK;
     }

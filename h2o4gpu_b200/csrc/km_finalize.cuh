@@ -615,6 +615,7 @@ __device__ __forceinline__ void split_table_row<float>(const SplitTable& tp, int
 // run_if: 0 = only when the M-step found no empty cluster, 1 = only when it found one (queued
 // behind the repair kernels), 2 = always.  The pair (0, 1) around the gated repair kernels lets the
 // stream decide on the device, so the host never waits for the count of empty clusters.
+// amb_limit: rows the E-step may list for the exact pass before a fit on rounded rows goes back to whole ones.
 template <typename T>
 __global__ void __launch_bounds__(128)
 close_kernel(const long long* __restrict__ gsums, const unsigned long long* __restrict__ gcounts,
@@ -624,7 +625,7 @@ close_kernel(const long long* __restrict__ gsums, const unsigned long long* __re
              double* __restrict__ shift_log, unsigned long long* __restrict__ changed_log,
              int* __restrict__ reloc_log, unsigned int* __restrict__ amb_log, int it,
              double* __restrict__ host_shift, unsigned long long* __restrict__ host_changed,
-             unsigned int* __restrict__ ticket, SplitTable tp) {
+             unsigned int* __restrict__ ticket, SplitTable tp, unsigned int amb_limit) {
   constexpr int NP = Fixed<T>::NP;
   // count_unit: weight of one unit of gcounts (1 for plain counts, a power of two for sample weights)
   const int n_empty = st->n_empty;
@@ -722,6 +723,7 @@ close_kernel(const long long* __restrict__ gsums, const unsigned long long* __re
     changed_log[it] = st->changed;
     reloc_log[it] = st->relocated;
     amb_log[it] = st->amb_count;
+    if (st->amb_count > amb_limit) st->full_rows = 1;
     st->amb_count = 0;
     if (host_shift) { *host_shift = red[0]; *host_changed = st->changed; }
     st->changed = 0;

@@ -151,7 +151,7 @@ int Engine<T>::launch_close(Shard<T>& s, int run_if, int it, double inv, bool us
                                            s.shift_k, s.st, s.Cd[cur ^ 1], run_if, weighted ? count_unit : 1.0,
                                            s.shift_log, s.changed_log, s.reloc_log, s.amb_log, it, &s.host_pin[0],
                                            reinterpret_cast<unsigned long long*>(&s.host_pin[1]), s.ticket,
-                                           split_table(s, use_tc));
+                                           split_table(s, use_tc), (unsigned int)(s.rows / 4));
   KM_CUDA(cudaGetLastError());
   ++launches;
   return KM_OK;
@@ -184,9 +184,9 @@ int Engine<T>::fit(int k_, int max_iter, double threshold, const T* init, int fl
   // the sorted pass do not carry weights); the incremental sums do
   const bool fused = smallk_ok(true) && !(flags & KM_FIT_FORCE_SPLIT) && !weighted;
   const bool use_tc = !fused && tc_ok(flags);
-  // the split copy of X (d = 64 tensor-core kernel without converter warps) costs about as much as
-  // sixteen iterations save
-  tc_split_build = max_iter >= 16 || (flags & KM_FIT_PRESPLIT);
+  // the fp16 copy of X (d = 64 tensor-core kernel without converter warps) takes the place of the row norms'
+  // pass and costs about as much more as one iteration saves
+  tc_split_build = max_iter >= 3 || (flags & KM_FIT_PRESPLIT);
   struct SplitBuildGuard { bool& f; ~SplitBuildGuard() { f = false; } } split_build_guard{tc_split_build};
   // incremental M-step (km_accumulate_delta.cuh): on unless the caller or the environment asks
   // for a full recomputation every iteration; a shard switches to it, on the device, in the

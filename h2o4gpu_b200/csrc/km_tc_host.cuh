@@ -56,20 +56,22 @@ struct Plan {
   float sx = 1.f, sb = 1.f;
   CUtensorMap tmX, tmBhi, tmBlo;
   bool ready = false;
-  // the rows split once into fp16 halves (d = 64): [rows][64] upper, then [rows][64] lower
+  // the rows rounded once to fp16 (d = 64), and per row |x|^2 and the length of what the rounding left out
   __half* xsplit = nullptr;
+  float2* xrowq = nullptr;
   size_t xsplit_cap = 0;
   const float* xsplit_of = nullptr;
   size_t xsplit_rows = 0;
   float xsplit_sx = 0.f;
   bool xsplit_failed = false;   // no memory for it: stay with the converting kernel
-  CUtensorMap tmXh, tmXl;
+  CUtensorMap tmXh;
 
   void release() {
-    km_free(bhi); km_free(blo); km_free(cn); km_free(xnorm); km_free(xsplit);
+    km_free(bhi); km_free(blo); km_free(cn); km_free(xnorm); km_free(xsplit); km_free(xrowq);
     bhi = blo = nullptr;
     cn = xnorm = nullptr;
     xsplit = nullptr;
+    xrowq = nullptr;
     xnorm_cap = xsplit_cap = 0;
     xnorm_of = xsplit_of = nullptr;
     ready = false;
@@ -109,8 +111,8 @@ inline int ensure_xnorm(Plan& pl, const float* X, size_t rows, int d, int num_sm
   return KM_OK;
 }
 
-// The split copy of X for the kernel variant without converter warps (d = 64): made when the
-// matrix, its size or the scale changed; costs one pass over X and as much memory again.
+// The fp16 copy of X for the kernel variant without converter warps (d = 64): made when the
+// matrix, its size or the scale changed; costs one pass over X and half as much memory again.
 inline bool presplit_enabled() {
   static const bool on = [] {
     const char* e = std::getenv("H2O4GPU_KM_TC_PRESPLIT");
@@ -125,20 +127,20 @@ inline bool ensure_xsplit(Plan& pl, const float* X, size_t rows, int d, float sx
   if (!allow_build) return false;   // a single pass (predict) does not pay for the split
   if (pl.xsplit_cap < rows) {
     km_free(pl.xsplit);
+    km_free(pl.xrowq);
     pl.xsplit = nullptr;
+    pl.xrowq = nullptr;
     pl.xsplit_cap = 0;
-    if (km_malloc(&pl.xsplit, rows * 64 * 2 * sizeof(__half)) != cudaSuccess) {
+    if (km_malloc(&pl.xsplit, rows * 64 * sizeof(__half)) != cudaSuccess ||
+        km_malloc(&pl.xrowq, rows * sizeof(float2)) != cudaSuccess) {
       cudaGetLastError();
       pl.xsplit_failed = true;
       return false;
     }
     pl.xsplit_cap = rows;
   }
-  __half* xh = pl.xsplit;
-  __half* xl = pl.xsplit + rows * 64;
-  split_rows_kernel<<<num_sms * 8, 256, 0, stream>>>(X, rows * 64, sx, xh, xl);
-  if (cudaGetLastError() != cudaSuccess || make_map(&pl.tmXh, xh, rows, 64, kBM, 2) != KM_OK ||
-      make_map(&pl.tmXl, xl, rows, 64, kBM, 2) != KM_OK) {
+  split_rows_kernel<<<num_sms * 8, 256, 0, stream>>>(X, rows, sx, pl.xsplit, pl.xrowq);
+  if (cudaGetLastError() != cudaSuccess || make_map(&pl.tmXh, pl.xsplit, rows, 64, kBM, 2) != KM_OK) {
     pl.xsplit_failed = true;
     return false;
   }
@@ -150,7 +152,6 @@ inline bool ensure_xsplit(Plan& pl, const float* X, size_t rows, int d, float sx
 
 inline int setup(Plan& pl, const float* X, size_t rows, int k, int d, int num_sms, cudaStream_t stream) {
   const int npad = (k + 15) / 16 * 16;
-  KM_TRY(ensure_xnorm(pl, X, rows, d, num_sms, stream));
   if (pl.ready && pl.k == k && pl.d == d && pl.x_base == X && pl.x_rows == rows) return KM_OK;
   if (!(pl.bhi && pl.k == k && pl.d == d)) {
     km_free(pl.bhi); km_free(pl.blo); km_free(pl.cn);
@@ -166,12 +167,12 @@ inline int setup(Plan& pl, const float* X, size_t rows, int k, int d, int num_sm
   KM_TRY(make_map(&pl.tmBlo, pl.blo, npad, 64, npad, 2));
   if (d == 32) {
     KM_CUDA(cudaFuncSetAttribute(assign_tc_kernel<32, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)smem_bytes(d, npad)));
+                                 (int)smem_bytes(d, npad, false)));
   } else {
     KM_CUDA(cudaFuncSetAttribute(assign_tc_kernel<64, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)smem_bytes(d, npad)));
+                                 (int)smem_bytes(d, npad, false)));
     KM_CUDA(cudaFuncSetAttribute(assign_tc_kernel<64, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)smem_bytes(d, npad)));
+                                 (int)smem_bytes(d, npad, true)));
   }
   pl.ready = true;
   return KM_OK;
@@ -209,28 +210,28 @@ constexpr float kTolRel = 1.9073486328125e-06f;
 inline float tol_rel_of(int d) { return kTolRel * (0.8f + (float)d / 200.0f); }
 inline float tol_floor_of(int d) { return 1.1920928955078125e-07f * std::sqrt((float)d); }
 
-inline int launch(Plan& pl, int* labels, IterState* st, bool count_changes, unsigned int* amb_rows, float tol_rel,
-                  int num_sms, cudaStream_t stream, unsigned int* moved_bits, uint4* amb_near,
-                  bool allow_split_build) {
+inline int launch(Plan& pl, int* labels, IterState* st, bool count_changes, unsigned int* amb_rows,
+                  unsigned int* amb_seg, float tol_rel, int num_sms, cudaStream_t stream, unsigned int* moved_bits,
+                  uint4* amb_near, bool allow_split_build, int* launches) {
   const size_t tiles = (pl.x_rows + kBM - 1) / kBM;
   if (tiles > 0x7fffffffULL / kBM) KM_FAIL(KM_EINVAL, "shard too large for the tensor-core kernel");
   const int grid = (int)std::min<size_t>(tiles, (size_t)num_sms);
+  const unsigned int seg_cap = (unsigned int)amb_seg_rows(pl.x_rows, num_sms);
   const bool pre = ensure_xsplit(pl, pl.x_base, pl.x_rows, pl.d, pl.sx, num_sms, stream, allow_split_build);
-  if (pl.d == 32)
-    assign_tc_kernel<32, false><<<grid, kThreads, smem_bytes(pl.d, pl.npad), stream>>>(
-        pl.tmX, pl.tmX, pl.tmBhi, pl.tmBlo, pl.cn, pl.xnorm, labels, pl.x_rows, (int)tiles, pl.npad, st,
-        count_changes ? 1 : 0, amb_rows, tol_rel, tol_floor_of(pl.d), pl.sx, pl.sx * pl.sb, count_changes ? moved_bits : nullptr,
-        amb_near, wait_limits().mbar_iters);
-  else if (pre)
-    assign_tc_kernel<64, true><<<grid, kThreads, smem_bytes(pl.d, pl.npad), stream>>>(
-        pl.tmXh, pl.tmXl, pl.tmBhi, pl.tmBlo, pl.cn, pl.xnorm, labels, pl.x_rows, (int)tiles, pl.npad, st,
-        count_changes ? 1 : 0, amb_rows, tol_rel, tol_floor_of(pl.d), pl.sx, pl.sx * pl.sb, count_changes ? moved_bits : nullptr,
-        amb_near, wait_limits().mbar_iters);
-  else
-    assign_tc_kernel<64, false><<<grid, kThreads, smem_bytes(pl.d, pl.npad), stream>>>(
-        pl.tmX, pl.tmX, pl.tmBhi, pl.tmBlo, pl.cn, pl.xnorm, labels, pl.x_rows, (int)tiles, pl.npad, st,
-        count_changes ? 1 : 0, amb_rows, tol_rel, tol_floor_of(pl.d), pl.sx, pl.sx * pl.sb, count_changes ? moved_bits : nullptr,
-        amb_near, wait_limits().mbar_iters);
+  if (!pre) KM_TRY(ensure_xnorm(pl, pl.x_base, pl.x_rows, pl.d, num_sms, stream));
+  auto go = [&](auto fn, const CUtensorMap& tmX, bool p) {
+    fn<<<grid, kThreads, smem_bytes(pl.d, pl.npad, p), stream>>>(
+        tmX, pl.tmBhi, pl.tmBlo, pl.cn, pl.xnorm, pl.xrowq, labels, pl.x_rows, (int)tiles, pl.npad, st,
+        count_changes ? 1 : 0, amb_rows, amb_seg, seg_cap, tol_rel, tol_floor_of(pl.d), pl.sx, pl.sx * pl.sb,
+        count_changes ? moved_bits : nullptr, amb_near, pre ? 1 : 0, wait_limits().mbar_iters);
+    ++*launches;
+  };
+  if (pl.d == 32) {
+    go(assign_tc_kernel<32, false>, pl.tmX, false);
+  } else {
+    if (pre) go(assign_tc_kernel<64, true>, pl.tmXh, true);
+    go(assign_tc_kernel<64, false>, pl.tmX, false);
+  }
   KM_CUDA(cudaGetLastError());
   return KM_OK;
 }
