@@ -56,7 +56,8 @@ __device__ __forceinline__ void mma884(double (&c)[2], double a, double b) {
 
 __global__ void __launch_bounds__(kThreads, 2)
 assign_kernel(const double* __restrict__ X, size_t n, int d, const double* __restrict__ C, int k,
-              const double* __restrict__ cnorm, int* __restrict__ labels, IterState* st) {
+              const double* __restrict__ cnorm, int* __restrict__ labels, IterState* st, const IterState* gate) {
+  if (gate && !gate->full_rows) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   double* stage = reinterpret_cast<double*>(smem_raw);   // [kStages][(BM + BN)][kPitch]
   __shared__ double s_best[kWarpsN][BM];
@@ -184,7 +185,7 @@ assign_kernel(const double* __restrict__ X, size_t n, int d, const double* __res
 }
 
 inline int launch(const double* X, size_t n, int d, const double* C, int k, const double* cnorm, int* labels,
-                  IterState* st, cudaStream_t stream) {
+                  IterState* st, cudaStream_t stream, const IterState* gate) {
   // per device, so set on every launch (cheap)
   KM_CUDA(cudaFuncSetAttribute(assign_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes));
   // without this the driver sizes the shared-memory carve-out for one CTA and only one is resident
@@ -192,7 +193,7 @@ inline int launch(const double* X, size_t n, int d, const double* C, int k, cons
   const size_t grid = (n + BM - 1) / BM;
   if (grid == 0) return KM_OK;
   if (grid > 0x7fffffffULL) KM_FAIL(KM_EINVAL, "shard too large for one launch");
-  assign_kernel<<<(unsigned)grid, kThreads, kSmemBytes, stream>>>(X, n, d, C, k, cnorm, labels, st);
+  assign_kernel<<<(unsigned)grid, kThreads, kSmemBytes, stream>>>(X, n, d, C, k, cnorm, labels, st, gate);
   KM_CUDA(cudaGetLastError());
   return KM_OK;
 }

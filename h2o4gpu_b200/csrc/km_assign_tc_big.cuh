@@ -52,22 +52,38 @@ inline size_t big_smem_bytes(int kpad) {
   return 1024 + Cf::kXBytes + (size_t)kBStages * Cf::kBBytes + (size_t)kpad * 4 + 3 * kBM * 4 + NBARS * 8 + 64;
 }
 
-// bh/bl: [kpad][DP] halves of -2 c * sb (zero padded), cn_pad[kpad] scaled |c|^2 (+inf padding),
-// cn_pad[kpad] = max |c|^2 (zeroed before the launch)
+// bh/bl: [kpad][DP] halves of -2 c * sb (zero padded; bl may be null), cn_pad[kpad] scaled |c|^2 (+inf padding),
+// cn_pad[kpad] = max |c|^2 (zeroed before the launch); eb (or null): cn_pad[kpad + 1] = the largest length of what
+// the upper halves of a centroid leave out (zeroed as well)
+template <typename T>
 __global__ void __launch_bounds__(256)
-big_prep_kernel(const float* __restrict__ C, const float* __restrict__ cnorm, int k, int d, int dp, int kpad,
+big_prep_kernel(const T* __restrict__ C, const T* __restrict__ cnorm, int k, int d, int dp, int kpad,
                 float sb, float sxsb, __half* __restrict__ bhi, __half* __restrict__ blo,
-                float* __restrict__ cn_pad) {
+                float* __restrict__ cn_pad, const float* eb) {
   const int j = blockIdx.x;
+  double left = 0;
   for (int t = threadIdx.x; t < dp; t += blockDim.x) {
-    float v = (j < k && t < d) ? -2.0f * C[(size_t)j * d + t] * sb : 0.0f;
-    const __half h = __float2half_rn(v);
+    const T v = (j < k && t < d) ? (T)-2 * C[(size_t)j * d + t] * (T)sb : (T)0;
+    const __half h = to_half(v);
+    const T r = v - (T)__half2float(h);   // exact
     bhi[(size_t)j * dp + t] = h;
-    blo[(size_t)j * dp + t] = __float2half_rn(v - __half2float(h));
+    if (blo) blo[(size_t)j * dp + t] = to_half(r);
+    left = fma((double)r, (double)r, left);
   }
   if (threadIdx.x == 0) {
-    cn_pad[j] = (j < k) ? cnorm[j] * sxsb : __int_as_float(0x7f800000);
-    if (j < k) atomicMax(reinterpret_cast<int*>(cn_pad + kpad), __float_as_int(cnorm[j]));
+    cn_pad[j] = (j < k) ? (float)cnorm[j] * sxsb : __int_as_float(0x7f800000);
+    if (j < k) atomicMax(reinterpret_cast<int*>(cn_pad + kpad), __float_as_int((float)cnorm[j]));
+  }
+  if (eb) {
+    __shared__ double part[8];
+    left = warp_sum(left);
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = left;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      double s = 0;
+      for (int w = 0; w < 8; ++w) s += part[w];
+      atomicMax(reinterpret_cast<int*>(cn_pad + kpad + 1), __float_as_int(1.0001f * (float)sqrt(s)));
+    }
   }
 }
 
@@ -86,9 +102,10 @@ template <int D>
 __global__ void __launch_bounds__(kBigThreads, 1)
 assign_tc_big_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmBhi,
                      const __grid_constant__ CUtensorMap tmBlo, const float* __restrict__ cn_pad,
-                     const float* __restrict__ xnorm, int* __restrict__ labels, size_t n, int n_tiles, int kpad,
-                     IterState* st, int count_changes, unsigned int* __restrict__ amb_rows, float tol_rel,
-                     float tol_floor, float sx, float sxsb, unsigned int wait_iters) {
+                     const float* __restrict__ xnorm, int xnorm_pitch, int* __restrict__ labels, size_t n, int n_tiles,
+                     int kpad, IterState* st, int count_changes, unsigned int* __restrict__ amb_rows, float tol_rel,
+                     float tol_floor, float sx, float sxsb, int gate, unsigned int wait_iters) {
+  if (gate && !st->full_rows) return;   // queued behind the one-product kernel: works only when that gave up
   using Cf = BigCfg<D>;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw_u32 = smem_u32(smem_raw);
@@ -317,7 +334,7 @@ assign_tc_big_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
       int old_label = -1;
       float xn = 0.f;
       if (grp == 0 && row < n) {
-        xn = xnorm[row];
+        xn = xnorm[row * (size_t)xnorm_pitch];
         if (count_changes) old_label = labels[row];
       }
       float rbest = kInf, rsecond = kInf;
@@ -409,6 +426,7 @@ assign_tc_big_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
 
   __syncthreads();
   if (tid == 0 && *abort_flag) atomicMax(&st->error, *abort_flag);
+  if (gate && tid == 0 && blockIdx.x == 0) st->pad_ready = 1;
   if (warp == 1) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)kTmemCols)

@@ -2,6 +2,7 @@
 // representation of the centroid sums, small device utilities.
 #pragma once
 
+#include <cuda_fp16.h>
 #include <algorithm>
 #include <cstdlib>
 #include <mutex>
@@ -268,6 +269,10 @@ __device__ __forceinline__ double warp_sum(double v) {
   return v;
 }
 
+// one rounding to fp16, to nearest
+__device__ __forceinline__ __half to_half(float v) { return __float2half_rn(v); }
+__device__ __forceinline__ __half to_half(double v) { return __double2half(v); }
+
 template <typename T> struct Inf;
 template <> struct Inf<float> { __device__ static float v() { return __int_as_float(0x7f800000); } };
 template <> struct Inf<double> { __device__ static double v() { return __longlong_as_double(0x7ff0000000000000LL); } };
@@ -280,8 +285,12 @@ struct IterState {
   int relocated;                // relocations done in the current M-step
   int error;                    // sticky device-side error word (0 = none)
   unsigned int amb_count;       // rows handed to the exact re-evaluation pass in the current E-step
-  unsigned int full_rows;       // 1: an E-step on rounded rows listed too many for the exact pass; the fit goes on with
-                                // the kernel that reads the whole rows (set by close_kernel, cleared when a fit begins)
+  unsigned int cand_count;      // rows the one-product kernel left to its exact pass in the current E-step
+  unsigned int cand_all;        // ... of which all chunks may hold the nearest centroid
+  unsigned int half_done;       // CTAs of the running one-product kernel that have finished (zero between launches)
+  unsigned int full_rows;       // 1: an E-step on rounded rows left too many open for the exact pass; the fit goes on
+                                // with the kernel that reads the whole rows (cleared when a fit begins, data is attached)
+  unsigned int pad_ready;       // 1: the padded copy those need for unaligned rows has been filled (cleared alike)
   double shift_sq;              // summed squared centroid shift of the current M-step
   double inertia;               // scratch for the inertia pass
 };

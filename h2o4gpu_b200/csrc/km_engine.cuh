@@ -97,6 +97,7 @@ struct Shard {
   int cc_major = 0;
   tc::Plan tcp;  // tensor-core path (float only)
   tcb::BigPlan tcbp;  // tensor-core path for large centroid tables
+  tch::HalfPlan tchp; // one-product kernel on rounded rows (large tables; float64)
   tcw::WidePlan tcwp; // tensor-core path for few centroids and wide rows
   tcs::StreamPlan tcsp;  // tensor-core path with both operands streamed: wide rows and many centroids, transform
   unsigned int* amb_rows = nullptr;  // rows handed to the exact re-evaluation pass
@@ -229,8 +230,10 @@ struct Engine : EngineBase {
   int poll_seq = 0;   // sequence number the finalize kernels publish to pinned memory
   bool tc_ok(int flags) const;
   // which tensor-core distance kernel labels this shape: 1 table resident (d 32/64, k <= 128), 2 table streamed
-  // (d <= 256), 3 few centroids and wide rows, 4 both operands streamed (wider rows, many centroids), 0 none
+  // (d <= 256), 3 few centroids and wide rows, 4 both operands streamed (wider rows, many centroids), 5 float64 rows
+  // rounded to fp16, 0 none
   int tc_kind() const {
+    if (!std::is_same<T, float>::value) return half_shape_ok() ? 5 : 0;
     if (tcw::wide_shape_ok(k, dtc())) return 3;
     if (d % 4 == 0 && tc::shape_ok(k, d)) return 1;
     if (tcb::big_shape_ok(k, dtc())) return 2;
@@ -241,7 +244,23 @@ struct Engine : EngineBase {
   // copy of the shard padded with zero columns to dtc() columns (built once per attached matrix; the exact pass,
   // the sums and everything else keep reading the rows as they are).
   int dtc() const { return (d + 3) / 4 * 4; }
-  int ensure_xpad(Shard<T>& s);
+  int ensure_xpad(Shard<T>& s, bool fill = true);
+  // Shapes the one-product kernel on rounded rows takes over (km_assign_tc_half.cuh).  It brings two more launches
+  // and, once per matrix, the rounding pass (6 d bytes per row in place of 4 d for the row norms), about 5 us per
+  // E-step in all: below 2e9 multiplications the three-term kernel takes less than twice that.  Rows that are not
+  // 16-byte aligned would cost that kernel a padded copy (12 d bytes per row), so they change over earlier; float64
+  // rows, where the alternative runs at 29 TFLOP/s, earlier still.
+  bool half_shape_ok() const {
+    static const bool on = [] {
+      const char* e = std::getenv("H2O4GPU_KM_TC_HALF");
+      return !(e && e[0] == '0');
+    }();
+    if (!on || d > tch::kMaxD || k <= 16 || k > tch::kMaxK) return false;
+    size_t rows = 0;
+    for (const auto& s : shards) rows = std::max(rows, s.rows);
+    const double work = (double)rows * k * d;
+    return std::is_same<T, float>::value ? work >= (d % 4 == 0 ? 2e9 : 5e8) : (d >= 8 && work >= 1e8);
+  }
   // list of the rows handed to the exact pass (cut into one segment per CTA for the small-table kernel, which
   // also leaves a mask of candidates per listed row)
   int ensure_amb(Shard<T>& s, bool near) {
@@ -272,8 +291,10 @@ struct Engine : EngineBase {
   double cbound = 0;                // bound on |centroid coordinate|: max(|x|, |initial centroids|)
 
   // launch helpers (device of the shard must be current)
+  // gate: the kernel returns at once unless full_rows is set there
   int launch_tiles(Shard<T>& s, const T* Xp, size_t nrows, int* labels, int mode, T* out, size_t ld_out,
-                   bool count_changes);
+                   bool count_changes, const IterState* gate = nullptr);
+  int launch_half(Shard<T>& s, bool count_changes);
   int launch_smallk(Shard<T>& s, bool update, T scale);
   // sums of the current labels into dst (default: the working array); with a gate the
   // kernels return at once when the incremental branch has the iteration
@@ -413,6 +434,7 @@ void Engine<T>::destroy() {
     }
     s.tcp.release();
     s.tcbp.release();
+    s.tchp.release();
     s.tcwp.release();
     s.tcsp.release();
     km_free(s.amb_rows); km_free(s.amb_near); km_free(s.amb_seg); km_free(s.amb_log); km_free(s.xpad);
@@ -451,6 +473,7 @@ int Engine<T>::attach_device(int local, const T* dX, size_t rows, size_t cols, s
   s.tcp.xsplit_of = nullptr;
   s.tcp.ready = false;
   s.tcbp.ready = false;
+  s.tchp.of = nullptr;
   s.tcwp.ready = false;
   s.tcsp.ready = false;
   s.xpad_of = nullptr;
@@ -464,6 +487,7 @@ int Engine<T>::attach_device(int local, const T* dX, size_t rows, size_t cols, s
     s.labels_cap = rows;
   }
   KM_CUDA(cudaMemsetAsync(s.labels, 0xff, rows * sizeof(int), s.stream));
+  KM_CUDA(cudaMemsetAsync(&s.st->full_rows, 0, 2 * sizeof(unsigned int), s.stream));   // and pad_ready
   return KM_OK;
 }
 
@@ -975,17 +999,17 @@ int Engine<T>::set_centroids(int k_, const T* host_c) {
 // ---- kernel dispatch -----------------------------------------------------------
 template <typename T, int BM, int BN, int BK, int TM, int TN>
 static int launch_tile_cfg(const T* X, size_t n, int d, const T* C, int k, const T* cnorm, int* labels,
-                           IterState* st, T* out, size_t ld_out, int mode, bool vec, cudaStream_t stream) {
+                           IterState* st, T* out, size_t ld_out, int mode, bool vec, cudaStream_t stream, const IterState* gate) {
   constexpr int V = VecOf<T>::N;
   constexpr int NT = (BM / TM) * (BN / TN);
   size_t grid = (n + BM - 1) / BM;
   if (grid > 0x7fffffffULL) KM_FAIL(KM_EINVAL, "shard too large for one launch");
   if (mode == MODE_ASSIGN) {
-    if (vec) tile_kernel<T, BM, BN, BK, TM, TN, V, MODE_ASSIGN><<<(unsigned)grid, NT, 0, stream>>>(X, n, d, C, k, cnorm, labels, st, out, ld_out);
-    else tile_kernel<T, BM, BN, BK, TM, TN, 1, MODE_ASSIGN><<<(unsigned)grid, NT, 0, stream>>>(X, n, d, C, k, cnorm, labels, st, out, ld_out);
+    if (vec) tile_kernel<T, BM, BN, BK, TM, TN, V, MODE_ASSIGN><<<(unsigned)grid, NT, 0, stream>>>(X, n, d, C, k, cnorm, labels, st, out, ld_out, gate);
+    else tile_kernel<T, BM, BN, BK, TM, TN, 1, MODE_ASSIGN><<<(unsigned)grid, NT, 0, stream>>>(X, n, d, C, k, cnorm, labels, st, out, ld_out, gate);
   } else {
-    if (vec) tile_kernel<T, BM, BN, BK, TM, TN, V, MODE_TRANSFORM><<<(unsigned)grid, NT, 0, stream>>>(X, n, d, C, k, cnorm, labels, st, out, ld_out);
-    else tile_kernel<T, BM, BN, BK, TM, TN, 1, MODE_TRANSFORM><<<(unsigned)grid, NT, 0, stream>>>(X, n, d, C, k, cnorm, labels, st, out, ld_out);
+    if (vec) tile_kernel<T, BM, BN, BK, TM, TN, V, MODE_TRANSFORM><<<(unsigned)grid, NT, 0, stream>>>(X, n, d, C, k, cnorm, labels, st, out, ld_out, gate);
+    else tile_kernel<T, BM, BN, BK, TM, TN, 1, MODE_TRANSFORM><<<(unsigned)grid, NT, 0, stream>>>(X, n, d, C, k, cnorm, labels, st, out, ld_out, gate);
   }
   KM_CUDA(cudaGetLastError());
   return KM_OK;
@@ -994,32 +1018,32 @@ static int launch_tile_cfg(const T* X, size_t n, int d, const T* C, int k, const
 template <typename T> struct TileCfg;
 template <> struct TileCfg<float> {
   static int go(const float* X, size_t n, int d, const float* C, int k, const float* cn, int* lab, IterState* st,
-                float* out, size_t ld, int mode, bool vec, cudaStream_t s) {
-    if (k <= 64) return launch_tile_cfg<float, 128, 64, 16, 8, 4>(X, n, d, C, k, cn, lab, st, out, ld, mode, vec, s);
-    return launch_tile_cfg<float, 128, 128, 16, 8, 8>(X, n, d, C, k, cn, lab, st, out, ld, mode, vec, s);
+                float* out, size_t ld, int mode, bool vec, cudaStream_t s, const IterState* gate) {
+    if (k <= 64) return launch_tile_cfg<float, 128, 64, 16, 8, 4>(X, n, d, C, k, cn, lab, st, out, ld, mode, vec, s, gate);
+    return launch_tile_cfg<float, 128, 128, 16, 8, 8>(X, n, d, C, k, cn, lab, st, out, ld, mode, vec, s, gate);
   }
 };
 template <> struct TileCfg<double> {
   static int go(const double* X, size_t n, int d, const double* C, int k, const double* cn, int* lab, IterState* st,
-                double* out, size_t ld, int mode, bool vec, cudaStream_t s) {
+                double* out, size_t ld, int mode, bool vec, cudaStream_t s, const IterState* gate) {
     // labels for more than a few centroids: the float64 matrix unit (km_assign_dmma.cuh)
     static const bool dmma_env = [] {
       const char* e = std::getenv("H2O4GPU_KM_DMMA");
       return !(e && e[0] == '0');
     }();
     if (dmma_env && mode == MODE_ASSIGN && vec && dmma::shape_ok(k, d) && (reinterpret_cast<uintptr_t>(C) & 15) == 0)
-      return dmma::launch(X, n, d, C, k, cn, lab, st, s);
-    return launch_tile_cfg<double, 64, 64, 16, 4, 4>(X, n, d, C, k, cn, lab, st, out, ld, mode, vec, s);
+      return dmma::launch(X, n, d, C, k, cn, lab, st, s, gate);
+    return launch_tile_cfg<double, 64, 64, 16, 4, 4>(X, n, d, C, k, cn, lab, st, out, ld, mode, vec, s, gate);
   }
 };
 
 template <typename T>
 int Engine<T>::launch_tiles(Shard<T>& s, const T* Xp, size_t nrows, int* labels, int mode, T* out,
-                            size_t ld_out, bool count_changes) {
+                            size_t ld_out, bool count_changes, const IterState* gate) {
   bool vec = (d % VecOf<T>::N == 0) && ((reinterpret_cast<uintptr_t>(Xp) & 15) == 0);
   ++launches;
   return TileCfg<T>::go(Xp, nrows, d, s.C[cur], k, s.cnorm, labels, count_changes ? s.st : nullptr, out, ld_out,
-                        mode, vec, s.stream);
+                        mode, vec, s.stream, gate);
 }
 
 template <typename T, int V>
@@ -1185,10 +1209,12 @@ int Engine<T>::launch_accumulate(Shard<T>& s, T scale, long long* dst, const uns
 // compute capability 10.x; everything else runs on the SIMT kernels.
 template <typename T>
 bool Engine<T>::tc_ok(int flags) const {
-  if (!std::is_same<T, float>::value || (flags & KM_FIT_FORCE_SIMT)) return false;
-  if (tc_kind() == 0) return false;
+  if (flags & KM_FIT_FORCE_SIMT) return false;
+  const int kind = tc_kind();
+  if (kind == 0) return false;
   for (const auto& s : shards) {
     if (s.cc_major != 10 || !s.x_checked) return false;
+    if (kind == 5) continue;
     if (d % 4 == 0) {
       if ((reinterpret_cast<uintptr_t>(s.X) & 15) != 0) return false;
     } else if (!(s.xpad && s.xpad_cap >= s.rows * (size_t)dtc())) {
@@ -1207,7 +1233,20 @@ bool Engine<T>::tc_ok(int flags) const {
 
 template <typename T>
 int Engine<T>::tc_refresh(Shard<T>& s) {
-  if constexpr (std::is_same<T, float>::value) {
+  const bool half = half_shape_ok() && (tc_kind() == 2 || tc_kind() == 5);
+  s.tchp.on = false;
+  if constexpr (std::is_same<T, double>::value) {
+    double xmax = 0;
+    for (const auto& sh : shards) xmax = std::max(xmax, sh.xmax);
+    if (!half || s.rows > 0xffffffffULL || !tc::pick_scales(xmax, std::max(xmax, cbound), &tc_sx, &tc_sb)) return KM_OK;
+    s.tchp.on = tch::half_rows<T>(s.tchp, s.X, s.rows, d, tc_sx, s.num_sms, s.stream, &launches);
+    if (!s.tchp.on) return KM_OK;   // no memory for the rounded rows: the float64 kernels
+    KM_TRY(tcb::big_tables(s.tcbp, k, d, false));
+    s.tcbp.sx = tc_sx;
+    s.tcbp.sb = tc_sb;
+    KM_TRY(tcb::big_prep(s.tcbp, s.C[cur], s.cnorm, s.stream));
+    ++launches;
+  } else {
     double xmax = 0;
     for (const auto& sh : shards) xmax = std::max(xmax, sh.xmax);
     if (!tc::pick_scales(xmax, std::max(xmax, cbound), &tc_sx, &tc_sb))
@@ -1215,7 +1254,8 @@ int Engine<T>::tc_refresh(Shard<T>& s) {
     if (s.rows > 0xffffffffULL) KM_FAIL(KM_EINVAL, "shard too large for the tensor-core kernel");
     KM_TRY(ensure_amb(s, tc_kind() == 1));
     const int kind = tc_kind();
-    if (d % 4 != 0) KM_TRY(ensure_xpad(s));
+    if (half) s.tchp.on = tch::half_rows<T>(s.tchp, s.X, s.rows, d, tc_sx, s.num_sms, s.stream, &launches);
+    if (d % 4 != 0) KM_TRY(ensure_xpad(s, !s.tchp.on));
     if (kind == 3) {
       KM_TRY(tc::ensure_xnorm(s.tcp, xtc(s), s.rows, dtc(), s.num_sms, s.stream));   // float4 loads: the aligned rows
       KM_TRY(tcw::wide_setup(s.tcwp, xtc(s), s.rows, k, d, dtc()));
@@ -1230,7 +1270,8 @@ int Engine<T>::tc_refresh(Shard<T>& s) {
       s.tcp.sb = tc_sb;
       KM_TRY(tc::prep(s.tcp, s.C[cur], s.cnorm, s.stream));
     } else {
-      KM_TRY(tc::ensure_xnorm(s.tcp, xtc(s), s.rows, dtc(), s.num_sms, s.stream));   // float4 loads: the aligned rows
+      if (!s.tchp.on)
+        KM_TRY(tc::ensure_xnorm(s.tcp, xtc(s), s.rows, dtc(), s.num_sms, s.stream));   // float4 loads: the aligned rows
       KM_TRY(tcb::big_setup(s.tcbp, xtc(s), s.rows, k, d, dtc()));
       s.tcbp.sx = tc_sx;
       s.tcbp.sb = tc_sb;
@@ -1243,7 +1284,8 @@ int Engine<T>::tc_refresh(Shard<T>& s) {
 
 template <typename T>
 __global__ void __launch_bounds__(256)
-pad_rows_kernel(const T* __restrict__ X, size_t rows, int d, int dp, T* __restrict__ out) {
+pad_rows_kernel(const T* __restrict__ X, size_t rows, int d, int dp, T* __restrict__ out, const IterState* gate) {
+  if (gate && (!gate->full_rows || gate->pad_ready)) return;
   const size_t total = rows * (size_t)dp;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
     const size_t r = i / dp;
@@ -1252,8 +1294,9 @@ pad_rows_kernel(const T* __restrict__ X, size_t rows, int d, int dp, T* __restri
   }
 }
 
+// fill = false: the copy is allocated only; the E-step's kernels fill it should they come to need it
 template <typename T>
-int Engine<T>::ensure_xpad(Shard<T>& s) {
+int Engine<T>::ensure_xpad(Shard<T>& s, bool fill) {
   if (s.xpad_of == s.X && s.xpad_rows == s.rows && s.xpad) return KM_OK;
   const size_t need = s.rows * (size_t)dtc();
   if (s.xpad_cap < need) {
@@ -1263,7 +1306,8 @@ int Engine<T>::ensure_xpad(Shard<T>& s) {
     KM_CUDA(km_malloc(&s.xpad, need * sizeof(T)));
     s.xpad_cap = need;
   }
-  pad_rows_kernel<T><<<s.num_sms * 16, 256, 0, s.stream>>>(s.X, s.rows, d, dtc(), s.xpad);
+  if (!fill) return KM_OK;
+  pad_rows_kernel<T><<<s.num_sms * 16, 256, 0, s.stream>>>(s.X, s.rows, d, dtc(), s.xpad, nullptr);
   KM_CUDA(cudaGetLastError());
   ++launches;
   s.xpad_of = s.X;
@@ -1304,9 +1348,19 @@ int Engine<T>::launch_assign(Shard<T>& s, bool use_tc, bool count_changes) {
       return KM_OK;
     }
     if (use_tc && tc_kind() == 2) {
+      const bool half = s.tchp.on;
+      if (half) {
+        KM_TRY(launch_half(s, count_changes));
+        // behind it, gated on the device, the pass that needs no list of open rows
+        if (d % 4 != 0 && s.xpad_of != s.X) {
+          pad_rows_kernel<T><<<s.num_sms * 16, 256, 0, s.stream>>>(s.X, s.rows, d, dtc(), s.xpad, s.st);
+          KM_CUDA(cudaGetLastError());
+          ++launches;
+        }
+      }
       launches += 2;
-      KM_TRY(tcb::big_launch(s.tcbp, s.tcp.xnorm, s.labels, s.st, count_changes, s.amb_rows, tc::tol_rel_of(d), s.num_sms,
-                             s.stream));
+      KM_TRY(tcb::big_launch(s.tcbp, half ? &s.tchp.rowq->x : s.tcp.xnorm, half ? 2 : 1, s.labels, s.st, count_changes,
+                             s.amb_rows, tc::tol_rel_of(d), s.num_sms, s.stream, half));
       KM_TRY(launch_refine_big(s, count_changes));
       KM_CUDA(cudaGetLastError());
       return KM_OK;
@@ -1351,6 +1405,10 @@ int Engine<T>::launch_assign(Shard<T>& s, bool use_tc, bool count_changes) {
       return go(sks::assign_stream_kernel<16>);
     }
   }
+  if (use_tc && s.tchp.on) {   // float64 (float32 returned above)
+    KM_TRY(launch_half(s, count_changes));
+    return launch_tiles(s, s.X, s.rows, s.labels, MODE_ASSIGN, nullptr, 0, count_changes, s.st);
+  }
   if (smallk_ok(false)) {
     IterState* keep = s.st;
     if (!count_changes) s.st = nullptr;
@@ -1359,6 +1417,28 @@ int Engine<T>::launch_assign(Shard<T>& s, bool use_tc, bool count_changes) {
     return rc;
   }
   return launch_tiles(s, s.X, s.rows, s.labels, MODE_ASSIGN, nullptr, 0, count_changes);
+}
+
+// the one-product kernel and the exact pass over the rows it leaves open
+template <typename T>
+int Engine<T>::launch_half(Shard<T>& s, bool count_changes) {
+  KM_TRY(tch::half_launch(s.tchp, s.tcbp, s.labels, s.st, count_changes, tc::tol_rel_of(d), s.num_sms, s.stream));
+  const int grid = s.num_sms * 8, threads = tch::kExactWarps * 32, cc = count_changes ? 1 : 0;
+  if constexpr (std::is_same<T, double>::value) {
+    tch::half_exact_f64_kernel<<<grid, threads, 0, s.stream>>>(s.X, d, s.C[cur], k, s.tcbp.kpad, s.tchp.cand_near, s.st,
+                                                              s.labels, cc);
+  } else {
+    auto go = [&](auto fn) {
+      fn<<<grid, threads, 0, s.stream>>>(s.X, d, s.C[cur], s.Cd[cur], k, s.tcbp.kpad, s.tchp.cand_near, s.st, s.labels, cc);
+    };
+    const bool vec = vec_ok(s);
+    if (d <= 64) vec ? go(tch::half_exact_f32_kernel<2, true>) : go(tch::half_exact_f32_kernel<2, false>);
+    else if (d <= 128) vec ? go(tch::half_exact_f32_kernel<4, true>) : go(tch::half_exact_f32_kernel<4, false>);
+    else vec ? go(tch::half_exact_f32_kernel<8, true>) : go(tch::half_exact_f32_kernel<8, false>);
+  }
+  KM_CUDA(cudaGetLastError());
+  launches += 2;
+  return KM_OK;
 }
 
 template <typename T>

@@ -583,26 +583,36 @@ relocate_kernel(const T* __restrict__ X, size_t n, int d, const int* __restrict_
 // Where the split centroid table of the tensor-core distance kernels goes (null bhi: not used):
 // bhi / blo = fp16 halves of -2 c * sb, rows of `dp` halves (columns >= d zero), `npad` rows
 // (rows >= k zero); cn_pad[j] = |c_j|^2 * sxsb (+inf for padding rows), cn_pad[npad] = max |c_j|^2.
+// eb (or null): per centroid the length of what the upper halves leave out, its maximum in cn_pad[npad + 1].
 struct SplitTable {
   __half* bhi;
-  __half* blo;
+  __half* blo;   // null: upper halves only
   float* cn_pad;
+  float* eb;
   int npad, dp;
   float sb, sxsb;
+  // |c|^2 above which a centroid cannot be the nearest of any row: with R = sqrt(d) max|x| >= |x| and another
+  // centroid inside R (the mean of any cluster with members), |x - c| > 2 R once |c| > 3 R.  Such a centroid exists:
+  // a cluster that stays empty takes the unscaled sums of the largest one.  It enters the table as a padding row -
+  // its fp16 halves would overflow, and the error bounds of all rows grow with the longest centroid.
+  float far_sq;
 };
 
+// returns this thread's share of the squared length of what the upper halves leave out
 template <typename T>
-__device__ __forceinline__ void split_table_row(const SplitTable& tp, int j, int d, const T* c_row, T cn) {}
-template <>
-__device__ __forceinline__ void split_table_row<float>(const SplitTable& tp, int j, int d, const float* c_row,
-                                                       float cn) {
+__device__ __forceinline__ double split_table_row(const SplitTable& tp, int j, int d, const T* c_row, T cn) {
+  double left = 0;
+  const bool far = (float)cn > tp.far_sq;
   for (int t = threadIdx.x; t < tp.dp; t += blockDim.x) {
-    const float v = (t < d) ? -2.0f * c_row[t] * tp.sb : 0.0f;
-    const __half h = __float2half_rn(v);
+    const T v = (t < d && !far) ? (T)-2 * c_row[t] * (T)tp.sb : (T)0;
+    const __half h = to_half(v);
+    const T r = v - (T)__half2float(h);   // exact
     tp.bhi[(size_t)j * tp.dp + t] = h;
-    tp.blo[(size_t)j * tp.dp + t] = __float2half_rn(v - __half2float(h));
+    if (tp.blo) tp.blo[(size_t)j * tp.dp + t] = to_half(r);
+    left = fma((double)r, (double)r, left);
   }
-  if (threadIdx.x == 0) tp.cn_pad[j] = cn * tp.sxsb;
+  if (threadIdx.x == 0) tp.cn_pad[j] = far ? __int_as_float(0x7f800000) : (float)cn * tp.sxsb;
+  return left;
 }
 
 // One CTA per cluster closes an M-step: mean of the cluster in double -> T (inv = 2^-(sa+15) turns
@@ -679,7 +689,13 @@ close_kernel(const long long* __restrict__ gsums, const unsigned long long* __re
   }
   if (tp.bhi != nullptr) {
     __syncthreads();   // the row of C_new written above is read back by other threads
-    split_table_row<T>(tp, j, d, C_new + (size_t)j * d, cn);
+    const double left = split_table_row<T>(tp, j, d, C_new + (size_t)j * d, cn);
+    if (tp.eb != nullptr) {
+      const double w = warp_sum(left);
+      if ((threadIdx.x & 31) == 0) red_n[threadIdx.x >> 5] = w;
+      __syncthreads();
+      if (threadIdx.x == 0) tp.eb[j] = 1.0001f * (float)sqrt(red_n[0] + red_n[1] + red_n[2] + red_n[3]);
+    }
   }
   // ---- the last CTA closes the iteration ----
   __threadfence();
@@ -691,18 +707,25 @@ close_kernel(const long long* __restrict__ gsums, const unsigned long long* __re
   __shared__ double red[128];
   __shared__ float redm[128];
   double s = 0;
-  float m = 0.f;
+  float m = 0.f, meb = 0.f;
   for (int c = threadIdx.x; c < k; c += 128) {
     s += __ldcg(shift_k + c);
-    if (tp.bhi != nullptr) m = fmaxf(m, (float)__ldcg(cnorm + c));
+    if (tp.bhi != nullptr) {
+      const float cn_c = (float)__ldcg(cnorm + c);
+      if (!(cn_c > tp.far_sq)) m = fmaxf(m, cn_c);
+    }
+    if (tp.eb != nullptr) meb = fmaxf(meb, __ldcg(tp.eb + c));
   }
+  __shared__ float rede[128];
   red[threadIdx.x] = s;
   redm[threadIdx.x] = m;
+  rede[threadIdx.x] = meb;
   __syncthreads();
   for (int o = 64; o > 0; o >>= 1) {
     if (threadIdx.x < o) {
       red[threadIdx.x] += red[threadIdx.x + o];
       redm[threadIdx.x] = fmaxf(redm[threadIdx.x], redm[threadIdx.x + o]);
+      rede[threadIdx.x] = fmaxf(rede[threadIdx.x], rede[threadIdx.x + o]);
     }
     __syncthreads();
   }
@@ -710,11 +733,12 @@ close_kernel(const long long* __restrict__ gsums, const unsigned long long* __re
     for (int r = k; r < tp.npad; ++r) {
       for (int t = threadIdx.x; t < tp.dp; t += 128) {
         tp.bhi[(size_t)r * tp.dp + t] = __float2half_rn(0.f);
-        tp.blo[(size_t)r * tp.dp + t] = __float2half_rn(0.f);
+        if (tp.blo) tp.blo[(size_t)r * tp.dp + t] = __float2half_rn(0.f);
       }
       if (threadIdx.x == 0) tp.cn_pad[r] = __int_as_float(0x7f800000);
     }
     if (threadIdx.x == 0) tp.cn_pad[tp.npad] = redm[0];
+    if (threadIdx.x == 0 && tp.eb != nullptr) tp.cn_pad[tp.npad + 1] = rede[0];
   }
   if (threadIdx.x == 0) {
     *ticket = 0;
@@ -722,9 +746,10 @@ close_kernel(const long long* __restrict__ gsums, const unsigned long long* __re
     shift_log[it] = red[0];
     changed_log[it] = st->changed;
     reloc_log[it] = st->relocated;
-    amb_log[it] = st->amb_count;
+    amb_log[it] = st->amb_count + st->cand_count;
     if (st->amb_count > amb_limit) st->full_rows = 1;
     st->amb_count = 0;
+    st->cand_count = 0;
     if (host_shift) { *host_shift = red[0]; *host_changed = st->changed; }
     st->changed = 0;
   }

@@ -51,7 +51,7 @@ int Engine<T>::assign_all(int flags) {
     const bool use_tc = tc_ok(flags) && (!smallk_ok(false) || tc_kind() == 3);
     if (use_tc) {
       KM_TRY(tc_refresh(s));
-      KM_CUDA(cudaMemsetAsync(&s.st->amb_count, 0, sizeof(unsigned int), s.stream));
+      KM_CUDA(cudaMemsetAsync(&s.st->amb_count, 0, 2 * sizeof(unsigned int), s.stream));   // and cand_count
     }
     KM_TRY(launch_assign(s, use_tc, false));
   }
@@ -130,17 +130,21 @@ int Engine<T>::relocate_multi(double scale, int seq, int* n_empty) {
 
 template <typename T>
 SplitTable Engine<T>::split_table(Shard<T>& s, bool use_tc) {
-  SplitTable tp{nullptr, nullptr, nullptr, 0, 0, 0.f, 0.f};
+  double xmax = 0;
+  for (const auto& sh : shards) xmax = std::max(xmax, sh.xmax);
+  const float far_sq = (float)(9.1 * d * xmax * xmax);
+  SplitTable tp{nullptr, nullptr, nullptr, nullptr, 0, 0, 0.f, 0.f, far_sq};
   if constexpr (std::is_same<T, float>::value) {
     if (use_tc && tc_kind() == 4)
-      tp = SplitTable{s.tcsp.bhi, s.tcsp.blo, s.tcsp.cn, s.tcsp.kpad, s.tcsp.dp, s.tcsp.sb, s.tcsp.sx * s.tcsp.sb};
+      tp = SplitTable{s.tcsp.bhi, s.tcsp.blo, s.tcsp.cn, nullptr, s.tcsp.kpad, s.tcsp.dp, s.tcsp.sb, s.tcsp.sx * s.tcsp.sb, far_sq};
     else if (use_tc && tc_kind() == 3)
-      tp = SplitTable{s.tcwp.bhi, s.tcwp.blo, s.tcwp.cn, tcw::kNPad, s.tcwp.dp, s.tcwp.sb, s.tcwp.sx * s.tcwp.sb};
+      tp = SplitTable{s.tcwp.bhi, s.tcwp.blo, s.tcwp.cn, nullptr, tcw::kNPad, s.tcwp.dp, s.tcwp.sb, s.tcwp.sx * s.tcwp.sb, far_sq};
     else if (use_tc && tc_kind() == 1)
-      tp = SplitTable{s.tcp.bhi, s.tcp.blo, s.tcp.cn, s.tcp.npad, 64, s.tcp.sb, s.tcp.sx * s.tcp.sb};
-    else if (use_tc)
-      tp = SplitTable{s.tcbp.bhi, s.tcbp.blo, s.tcbp.cn, s.tcbp.kpad, s.tcbp.dp, s.tcbp.sb, s.tcbp.sx * s.tcbp.sb};
+      tp = SplitTable{s.tcp.bhi, s.tcp.blo, s.tcp.cn, nullptr, s.tcp.npad, 64, s.tcp.sb, s.tcp.sx * s.tcp.sb, far_sq};
   }
+  if (!tp.bhi && use_tc && (tc_kind() == 2 || s.tchp.on))
+    tp = SplitTable{s.tcbp.bhi, s.tcbp.blo, s.tcbp.cn, s.tcbp.eb, s.tcbp.kpad, s.tcbp.dp, s.tcbp.sb,
+                    s.tcbp.sx * s.tcbp.sb, far_sq};
   return tp;
 }
 

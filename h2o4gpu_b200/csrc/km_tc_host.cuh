@@ -247,7 +247,8 @@ namespace tcb {
 struct BigPlan {
   __half* bhi = nullptr;
   __half* blo = nullptr;
-  float* cn = nullptr;
+  float* cn = nullptr;     // [kpad] scaled |c|^2, [kpad] max |c|^2, [kpad + 1] longest remainder of the upper halves
+  float* eb = nullptr;     // per centroid: length of what its upper halves leave out
   int kpad = 0, k = 0, d = 0, dp = 0;
   const float* x_base = nullptr;
   size_t x_rows = 0;
@@ -255,9 +256,9 @@ struct BigPlan {
   CUtensorMap tmX, tmBhi, tmBlo;
   bool ready = false;
   void release() {
-    km_free(bhi); km_free(blo); km_free(cn);
+    km_free(bhi); km_free(blo); km_free(cn); km_free(eb);
     bhi = blo = nullptr;
-    cn = nullptr;
+    cn = eb = nullptr;
     ready = false;
   }
 };
@@ -276,22 +277,30 @@ inline int big_set_attr(int kpad) {
   return KM_OK;
 }
 
-// ldx: row pitch of X in elements (d, or d rounded up to four for the padded copy of unaligned rows)
-inline int big_setup(BigPlan& pl, const float* X, size_t rows, int k, int d, int ldx) {
+// the operand table: upper and lower halves (float32) or upper halves only (float64)
+inline int big_tables(BigPlan& pl, int k, int d, bool lower) {
   const int kpad = (k + kNT - 1) / kNT * kNT;
   const int dv = big_variant(d);
   const int dp = dv < 64 ? 64 : dv;
-  if (pl.ready && pl.k == k && pl.d == d && pl.x_base == X && pl.x_rows == rows) return KM_OK;
-  if (!(pl.bhi && pl.k == k && pl.d == d)) {
-    pl.release();
-    KM_CUDA(km_malloc(&pl.bhi, (size_t)kpad * dp * sizeof(__half)));
-    KM_CUDA(km_malloc(&pl.blo, (size_t)kpad * dp * sizeof(__half)));
-    KM_CUDA(km_malloc(&pl.cn, (size_t)(kpad + 1) * sizeof(float)));
-  }
-  pl.kpad = kpad; pl.k = k; pl.d = d; pl.dp = dp; pl.x_base = X; pl.x_rows = rows;
-  KM_TRY(tc::make_map(&pl.tmX, X, rows, ldx, kBM, 4));
+  if (pl.eb && pl.k == k && pl.d == d) return KM_OK;
+  pl.release();
+  KM_CUDA(km_malloc(&pl.bhi, (size_t)kpad * dp * sizeof(__half)));
+  if (lower) KM_CUDA(km_malloc(&pl.blo, (size_t)kpad * dp * sizeof(__half)));
+  KM_CUDA(km_malloc(&pl.cn, (size_t)(kpad + 2) * sizeof(float)));
+  KM_CUDA(km_malloc(&pl.eb, (size_t)kpad * sizeof(float)));
+  pl.kpad = kpad; pl.k = k; pl.d = d; pl.dp = dp;
   KM_TRY(tc::make_map(&pl.tmBhi, pl.bhi, kpad, dp, kNT, 2));
-  KM_TRY(tc::make_map(&pl.tmBlo, pl.blo, kpad, dp, kNT, 2));
+  if (lower) KM_TRY(tc::make_map(&pl.tmBlo, pl.blo, kpad, dp, kNT, 2));
+  return KM_OK;
+}
+
+// ldx: row pitch of X in elements (d, or d rounded up to four for the padded copy of unaligned rows)
+inline int big_setup(BigPlan& pl, const float* X, size_t rows, int k, int d, int ldx) {
+  KM_TRY(big_tables(pl, k, d, true));
+  if (pl.ready && pl.x_base == X && pl.x_rows == rows) return KM_OK;
+  const int kpad = pl.kpad, dv = big_variant(d);
+  pl.x_base = X; pl.x_rows = rows;
+  KM_TRY(tc::make_map(&pl.tmX, X, rows, ldx, kBM, 4));
   if (dv == 32) KM_TRY(big_set_attr<32>(kpad));
   else if (dv == 64) KM_TRY(big_set_attr<64>(kpad));
   else if (dv == 128) KM_TRY(big_set_attr<128>(kpad));
@@ -300,38 +309,145 @@ inline int big_setup(BigPlan& pl, const float* X, size_t rows, int k, int d, int
   return KM_OK;
 }
 
-inline int big_prep(BigPlan& pl, const float* C, const float* cnorm, cudaStream_t stream) {
-  KM_CUDA(cudaMemsetAsync(pl.cn + pl.kpad, 0, sizeof(float), stream));
-  big_prep_kernel<<<pl.kpad, 256, 0, stream>>>(C, cnorm, pl.k, pl.d, pl.dp, pl.kpad, pl.sb, pl.sx * pl.sb, pl.bhi,
-                                               pl.blo, pl.cn);
+template <typename T>
+inline int big_prep(BigPlan& pl, const T* C, const T* cnorm, cudaStream_t stream) {
+  KM_CUDA(cudaMemsetAsync(pl.cn + pl.kpad, 0, 2 * sizeof(float), stream));
+  big_prep_kernel<T><<<pl.kpad, 256, 0, stream>>>(C, cnorm, pl.k, pl.d, pl.dp, pl.kpad, pl.sb, pl.sx * pl.sb, pl.bhi,
+                                                  pl.blo, pl.cn, pl.eb);
   KM_CUDA(cudaGetLastError());
   return KM_OK;
 }
 
 template <int D>
-inline void big_launch_d(BigPlan& pl, const float* xnorm, int* labels, IterState* st, int count_changes,
-                         unsigned int* amb_rows, float tol_rel, int grid, int tiles, cudaStream_t stream) {
+inline void big_launch_d(BigPlan& pl, const float* xnorm, int xnorm_pitch, int* labels, IterState* st, int count_changes,
+                         unsigned int* amb_rows, float tol_rel, int grid, int tiles, cudaStream_t stream, int gate) {
   assign_tc_big_kernel<D><<<grid, kBigThreads, big_smem_bytes<D>(pl.kpad), stream>>>(
-      pl.tmX, pl.tmBhi, pl.tmBlo, pl.cn, xnorm, labels, pl.x_rows, tiles, pl.kpad, st, count_changes, amb_rows,
-      tol_rel, tc::tol_floor_of(pl.d), pl.sx, pl.sx * pl.sb, wait_limits().mbar_iters);
+      pl.tmX, pl.tmBhi, pl.tmBlo, pl.cn, xnorm, xnorm_pitch, labels, pl.x_rows, tiles, pl.kpad, st, count_changes,
+      amb_rows, tol_rel, tc::tol_floor_of(pl.d), pl.sx, pl.sx * pl.sb, gate, wait_limits().mbar_iters);
 }
 
-inline int big_launch(BigPlan& pl, const float* xnorm, int* labels, IterState* st, bool count_changes,
-                      unsigned int* amb_rows, float tol_rel, int num_sms, cudaStream_t stream) {
+// gate: the kernel returns at once unless the one-product kernel in front of it gave the pass up; xnorm_pitch: floats
+// from one row's |x|^2 to the next
+inline int big_launch(BigPlan& pl, const float* xnorm, int xnorm_pitch, int* labels, IterState* st, bool count_changes,
+                      unsigned int* amb_rows, float tol_rel, int num_sms, cudaStream_t stream, bool gate) {
   const size_t tiles = (pl.x_rows + kBM - 1) / kBM;
   if (tiles > 0x7fffffffULL / kBM) KM_FAIL(KM_EINVAL, "shard too large for the tensor-core kernel");
   const int grid = (int)std::min<size_t>(tiles, (size_t)num_sms);
   const int cc = count_changes ? 1 : 0;
   const int dv = big_variant(pl.d);
-  if (dv == 32) big_launch_d<32>(pl, xnorm, labels, st, cc, amb_rows, tol_rel, grid, (int)tiles, stream);
-  else if (dv == 64) big_launch_d<64>(pl, xnorm, labels, st, cc, amb_rows, tol_rel, grid, (int)tiles, stream);
-  else if (dv == 128) big_launch_d<128>(pl, xnorm, labels, st, cc, amb_rows, tol_rel, grid, (int)tiles, stream);
-  else big_launch_d<256>(pl, xnorm, labels, st, cc, amb_rows, tol_rel, grid, (int)tiles, stream);
+  if (dv == 32) big_launch_d<32>(pl, xnorm, xnorm_pitch, labels, st, cc, amb_rows, tol_rel, grid, (int)tiles, stream, gate ? 1 : 0);
+  else if (dv == 64) big_launch_d<64>(pl, xnorm, xnorm_pitch, labels, st, cc, amb_rows, tol_rel, grid, (int)tiles, stream, gate ? 1 : 0);
+  else if (dv == 128) big_launch_d<128>(pl, xnorm, xnorm_pitch, labels, st, cc, amb_rows, tol_rel, grid, (int)tiles, stream, gate ? 1 : 0);
+  else big_launch_d<256>(pl, xnorm, xnorm_pitch, labels, st, cc, amb_rows, tol_rel, grid, (int)tiles, stream, gate ? 1 : 0);
   KM_CUDA(cudaGetLastError());
   return KM_OK;
 }
 
 }  // namespace tcb
+}  // namespace km
+
+#include "km_assign_tc_half.cuh"
+
+namespace km {
+namespace tch {
+
+// What the one-product kernel keeps per matrix (the rounded rows) and per fit (the list of open rows); the centroid
+// table is that of the three-term kernel (tcb::BigPlan).
+struct HalfPlan {
+  __half* xh = nullptr;           // [rows][ldh]
+  float2* rowq = nullptr;         // [rows] |x|^2, length of the rounding's remainder
+  size_t xh_cap = 0, rowq_cap = 0;
+  const void* of = nullptr;       // matrix the rounded rows belong to (null: none)
+  size_t rows = 0;
+  int ldh = 0;
+  float sx = 0.f;
+  CUtensorMap tmX;
+  uint4* cand_near = nullptr;
+  unsigned int cand_cap = 0;
+  bool on = false;                // the current E-steps run on the rounded rows
+
+  void release() {
+    km_free(xh); km_free(rowq); km_free(cand_near);
+    xh = nullptr; rowq = nullptr; cand_near = nullptr;
+    xh_cap = rowq_cap = 0;
+    cand_cap = 0;
+    of = nullptr;
+    on = false;
+  }
+};
+
+template <typename P>
+inline bool half_grow(P** p, size_t* cap, size_t need) {
+  if (*cap >= need) return true;
+  km_free(*p);
+  *p = nullptr;
+  *cap = 0;
+  if (km_malloc(p, need * sizeof(P)) != cudaSuccess) { cudaGetLastError(); return false; }
+  *cap = need;
+  return true;
+}
+
+// Rounded rows of X (made when the matrix or the scale changed) and the candidate list.  False: no memory for
+// them, the caller stays with the kernels that read the rows as they are.
+template <typename T>
+inline bool half_rows(HalfPlan& pl, const T* X, size_t rows, int d, float sx, int num_sms, cudaStream_t stream,
+                      int* launches) {
+  const int ldh = (d + 7) / 8 * 8;
+  // a quarter of the rows: settling an open row costs about twice its share of the pass that needs no list
+  const size_t cap = std::max<size_t>(rows / 4, std::min<size_t>(rows, 4096));
+  if (pl.cand_cap < cap) {
+    size_t have = pl.cand_cap;
+    pl.cand_cap = 0;
+    if (!half_grow(&pl.cand_near, &have, cap)) return false;
+    pl.cand_cap = (unsigned int)cap;
+  }
+  if (pl.of == X && pl.rows == rows && pl.sx == sx && pl.ldh == ldh) return true;
+  pl.of = nullptr;
+  if (!half_grow(&pl.xh, &pl.xh_cap, rows * (size_t)ldh) || !half_grow(&pl.rowq, &pl.rowq_cap, rows)) return false;
+  int lpr = 1;
+  while (lpr < 32 && lpr * 4 < ldh) lpr *= 2;
+  if (d % 4 == 0 && (reinterpret_cast<uintptr_t>(X) & 15) == 0)
+    half_rows_kernel<T, true><<<num_sms * 8, 256, 0, stream>>>(X, rows, d, ldh, lpr, sx, pl.xh, pl.rowq);
+  else
+    half_rows_kernel<T, false><<<num_sms * 8, 256, 0, stream>>>(X, rows, d, ldh, lpr, sx, pl.xh, pl.rowq);
+  if (cudaGetLastError() != cudaSuccess || tc::make_map(&pl.tmX, pl.xh, rows, ldh, kBM, 2) != KM_OK) return false;
+  ++*launches;
+  pl.of = X;
+  pl.rows = rows;
+  pl.sx = sx;
+  pl.ldh = ldh;
+  return true;
+}
+
+template <int P>
+inline int half_launch_p(HalfPlan& pl, tcb::BigPlan& tb, int* labels, IterState* st, bool count_changes, float tol_rel,
+                         int num_sms, cudaStream_t stream) {
+  const size_t n_sub = (pl.rows + kBM - 1) / kBM;
+  const int grid = (int)std::min<size_t>(n_sub, (size_t)num_sms);
+  const size_t smem = half_smem_bytes(tb.d, tb.kpad);
+  KM_CUDA(cudaFuncSetAttribute(assign_tc_half_kernel<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  // rows whose candidates cannot be told apart by chunk cost k / 32 times more in the exact pass; what takes over
+  // costs three times the one-product pass for float32 rows and forty times as much for float64 ones
+  const unsigned int all_limit = (unsigned int)std::max<size_t>(64, tb.blo ? pl.rows / 64 : pl.rows / 8);
+  assign_tc_half_kernel<P><<<grid, kHalfThreads, smem, stream>>>(
+      pl.tmX, tb.tmBhi, tb.cn, pl.rowq, labels, pl.rows, (int)n_sub, tb.kpad, (tb.d + 15) / 16, st,
+      count_changes ? 1 : 0, pl.cand_near, pl.cand_cap, all_limit, tol_rel, tc::tol_floor_of(tb.d),
+      tb.sx, tb.sx * tb.sb, wait_limits().mbar_iters);
+  KM_CUDA(cudaGetLastError());
+  return KM_OK;
+}
+
+inline int half_launch(HalfPlan& pl, tcb::BigPlan& tb, int* labels, IterState* st, bool count_changes, float tol_rel,
+                       int num_sms, cudaStream_t stream) {
+  switch (panels_of(tb.d)) {
+    case 1: return half_launch_p<1>(pl, tb, labels, st, count_changes, tol_rel, num_sms, stream);
+    case 2: return half_launch_p<2>(pl, tb, labels, st, count_changes, tol_rel, num_sms, stream);
+    case 3: return half_launch_p<3>(pl, tb, labels, st, count_changes, tol_rel, num_sms, stream);
+    default: return half_launch_p<4>(pl, tb, labels, st, count_changes, tol_rel, num_sms, stream);
+  }
+}
+
+}  // namespace tch
 }  // namespace km
 
 #include "km_assign_tc_wide.cuh"
@@ -395,8 +511,8 @@ inline int wide_setup(WidePlan& pl, const float* X, size_t rows, int k, int d, i
 
 inline int wide_prep(WidePlan& pl, const float* C, const float* cnorm, cudaStream_t stream) {
   KM_CUDA(cudaMemsetAsync(pl.cn + kNPad, 0, sizeof(float), stream));
-  tcb::big_prep_kernel<<<kNPad, 256, 0, stream>>>(C, cnorm, pl.k, pl.d, pl.dp, kNPad, pl.sb, pl.sx * pl.sb, pl.bhi,
-                                                  pl.blo, pl.cn);
+  tcb::big_prep_kernel<float><<<kNPad, 256, 0, stream>>>(C, cnorm, pl.k, pl.d, pl.dp, kNPad, pl.sb, pl.sx * pl.sb,
+                                                         pl.bhi, pl.blo, pl.cn, nullptr);
   KM_CUDA(cudaGetLastError());
   return KM_OK;
 }
@@ -479,8 +595,8 @@ inline int stream_setup(StreamPlan& pl, const float* X, size_t rows, int k, int 
 
 inline int stream_prep(StreamPlan& pl, const float* C, const float* cnorm, cudaStream_t stream) {
   KM_CUDA(cudaMemsetAsync(pl.cn + pl.kpad, 0, sizeof(float), stream));
-  tcb::big_prep_kernel<<<pl.kpad, 256, 0, stream>>>(C, cnorm, pl.k, pl.d, pl.dp, pl.kpad, pl.sb, pl.sx * pl.sb, pl.bhi,
-                                                   pl.blo, pl.cn);
+  tcb::big_prep_kernel<float><<<pl.kpad, 256, 0, stream>>>(C, cnorm, pl.k, pl.d, pl.dp, pl.kpad, pl.sb, pl.sx * pl.sb,
+                                                          pl.bhi, pl.blo, pl.cn, nullptr);
   KM_CUDA(cudaGetLastError());
   return KM_OK;
 }

@@ -64,7 +64,8 @@ template <typename T, int BM, int BN, int BK, int TM, int TN, int VEC, int MODE>
 __global__ void __launch_bounds__((BM / TM) * (BN / TN))
 tile_kernel(const T* __restrict__ X, size_t n, int d, const T* __restrict__ C, int k,
             const T* __restrict__ cnorm, int* __restrict__ labels, IterState* st,
-            T* __restrict__ out, size_t ld_out) {
+            T* __restrict__ out, size_t ld_out, const IterState* gate) {
+  if (gate && !gate->full_rows) return;
   constexpr int NTX = BN / TN;
   constexpr int NTY = BM / TM;
   constexpr int NT = NTX * NTY;

@@ -1351,3 +1351,73 @@ def test_random_shapes_one_step_matches_oracle(eng, n, d, k):
     h.assign()
     assert np.array_equal(h.labels(), lab2)
     h.close()
+
+
+# ---- one fp16 product per (row, centroid) with a proven bound, exact pass over the open rows ----
+def _nearest_gap(X, C, labels):
+    """Largest excess of a row's labelled squared distance over its smallest one, and the rows whose label is not the
+    lowest index among exactly equal smallest distances; direct differences in float64 for the few that differ."""
+    C = C.astype(np.float64)
+    cn = (C * C).sum(1)
+    wrong = 0
+    for s in range(0, X.shape[0], 8192):
+        x = X[s:s + 8192].astype(np.float64)
+        lab = labels[s:s + 8192]
+        near = (cn[None] - 2 * x @ C.T).argmin(1)
+        for i in np.flatnonzero(near != lab):
+            dist = ((x[i] - C) ** 2).sum(1)
+            wrong += int(dist.argmin() != lab[i])
+    return wrong
+
+
+# (rows, columns, centroids): widths around the 16-column MMA step and the 64-column panel, one to four panels,
+# unaligned rows, 128-centroid tiles with one and with 127 padding columns, row tiles that leave a CTA one tile or an
+# odd number of them; all above the size from which the kernel is used
+@pytest.mark.parametrize("dtype,n,d,k", [
+    (np.float32, 152_000, 64, 257), (np.float32, 18_945, 128, 1025), (np.float32, 38_017, 33, 1000),
+    (np.float32, 37_900, 129, 500), (np.float32, 20_000, 256, 640), (np.float32, 11_111, 193, 384),
+    (np.float32, 300_001, 50, 37), (np.float64, 20_001, 17, 500), (np.float64, 129, 256, 4000),
+    (np.float64, 9_600, 65, 513), (np.float64, 70_000, 256, 17)])
+@pytest.mark.parametrize("data", ["clusters", "close", "equal"])
+def test_one_product_kernel_labels_are_the_float64_argmin(eng, dtype, n, d, k, data):
+    """Labels of the kernel that forms one fp16 product per pair equal the float64 argmin, ties to the lowest index:
+    on clusters with several centroids each (some rows open, a few candidates each), on centroids so close together
+    that the bound leaves every row open (the pass goes back to the kernel behind it) and with every centroid present
+    several times (exact ties, candidates in more chunks than are recorded).  Incremental and full sums of a fit agree
+    bit for bit, so the label changes are counted right."""
+    rng = np.random.default_rng(n + d * 31 + k)
+    if data == "close":
+        X = (3.0 + 1e-3 * rng.standard_normal((n, d))).astype(dtype)
+    else:
+        centers = rng.uniform(-6, 6, (max(k // 3, 5), d))
+        X = (centers[rng.integers(0, centers.shape[0], n)] + rng.standard_normal((n, d))).astype(dtype)
+    C = X[np.sort(rng.choice(n, k, replace=n < k))].copy()
+    if data == "equal":
+        C = C[rng.integers(0, max(k // 6, 2), k)].copy()
+    h = eng.ResidentKMeans(dtype=dtype)
+    h.upload(X)
+    h.fit(C, 0)
+    assert h.stats()["path"] == 3
+    assert _nearest_gap(X, C, h.labels()) == 0
+    if data != "equal":
+        h.fit(C, 3)
+        got = h.centroids(), h.labels()
+        assert _nearest_gap(X, got[0], got[1]) == 0
+        h.fit(C, 3, flags=eng.FIT_FULL_SUMS)
+        assert np.array_equal(got[0], h.centroids()) and np.array_equal(got[1], h.labels())
+    h.close()
+
+
+def test_one_product_kernel_with_a_cluster_that_stays_empty(eng):
+    """More centroids than distinct rows: clusters that cannot be repaired take the unscaled sums of the largest one,
+    a point far outside the data whose fp16 operand would overflow.  The other labels stay the float64 argmin."""
+    rng = np.random.default_rng(5)
+    pts = rng.uniform(-5, 5, (300, 128))
+    for dtype in (np.float32, np.float64):
+        X = pts[rng.integers(0, 300, 40_000)].astype(dtype)
+        C = X[rng.choice(40_000, 500, replace=False)].copy()
+        h = eng.ResidentKMeans(dtype=dtype)
+        h.upload(X)
+        h.fit(C, 2)
+        assert _nearest_gap(X, h.centroids(), h.labels()) == 0
+        h.close()
