@@ -15,6 +15,7 @@
 #include <memory>
 #include <atomic>
 #include <mutex>
+#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -595,8 +596,12 @@ inline bool dispatch_dtype(int dt, F&& f) {
 // Replaces the pageable thrust::host_vector staging of copy_data (src/gpu/kmeans/kmeans_h2o4gpu.h:24-42).
 struct StagePool {
   static constexpr size_t kPiece = (size_t)4 << 20;
-  std::mutex busy;                 // one staged upload at a time
+  std::mutex busy;                 // one staged copy at a time
   std::vector<void*> bufs;
+  // a worker's stream and events, kept like the buffers: creating a stream takes about 0.6 ms under the driver's
+  // lock, which let the last of 14 workers begin when a quarter gigabyte was already through
+  struct Lane { cudaStream_t st = nullptr; cudaEvent_t ev[2] = {nullptr, nullptr}; };
+  std::map<int, std::vector<Lane>> lanes;   // by device
   static StagePool& get() {
     static StagePool* p = new StagePool();   // never destroyed: the CUDA runtime may be gone at exit
     return *p;
@@ -612,7 +617,45 @@ struct StagePool {
     }
     return KM_OK;
   }
+  // lanes of the device that is current; false: none to be had
+  bool ensure_lanes(int dev, size_t count) {
+    std::vector<Lane>& v = lanes[dev];
+    while (v.size() < count) {
+      Lane l;
+      if (cudaStreamCreateWithFlags(&l.st, cudaStreamNonBlocking) != cudaSuccess ||
+          cudaEventCreateWithFlags(&l.ev[0], cudaEventDisableTiming) != cudaSuccess ||
+          cudaEventCreateWithFlags(&l.ev[1], cudaEventDisableTiming) != cudaSuccess) {
+        cudaGetLastError();
+        destroy(l);
+        return false;
+      }
+      v.push_back(l);
+    }
+    return true;
+  }
+  static void destroy(Lane& l) {
+    for (auto& e : l.ev) if (e) cudaEventDestroy(e);
+    if (l.st) cudaStreamDestroy(l.st);
+  }
+  // everything back to the system, unless a copy is running
+  void trim() {
+    std::unique_lock<std::mutex> lock(busy, std::try_to_lock);
+    if (!lock.owns_lock()) return;
+    for (auto& kv : lanes) {
+      DevGuard g(kv.first);
+      for (auto& l : kv.second) destroy(l);
+    }
+    lanes.clear();
+    for (void* b : bufs) cudaFreeHost(b);
+    bufs.clear();
+  }
 };
+inline int stage_workers(size_t g) {
+  // a single core copies far less than the bus carries (about 4 GB/s against 55 GB/s on the hosts measured), so
+  // nearly all of them are put to work
+  const unsigned hw = std::max(3u, std::thread::hardware_concurrency());
+  return (int)std::max<size_t>(1, std::min<size_t>(14, hw - 2) / g);
+}
 
 inline bool host_pointer_is_pageable(const void* p) {
   cudaPointerAttributes a;
@@ -625,13 +668,11 @@ inline bool host_pointer_is_pageable(const void* p) {
 
 // one worker: pieces first, first + stride, ... of the byte range [src, src + bytes) of one shard
 inline void stage_worker(int dev, const unsigned char* src, unsigned char* dst, size_t bytes, size_t first,
-                         size_t stride, void* buf0, void* buf1, std::atomic<int>* err) {
-  cudaStream_t st = nullptr;
-  cudaEvent_t ev[2] = {nullptr, nullptr};
+                         size_t stride, void* buf0, void* buf1, StagePool::Lane lane, std::atomic<int>* err) {
+  cudaStream_t st = lane.st;
+  cudaEvent_t* ev = lane.ev;
   void* buf[2] = {buf0, buf1};
-  bool ok = cudaSetDevice(dev) == cudaSuccess && cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) == cudaSuccess &&
-            cudaEventCreateWithFlags(&ev[0], cudaEventDisableTiming) == cudaSuccess &&
-            cudaEventCreateWithFlags(&ev[1], cudaEventDisableTiming) == cudaSuccess;
+  bool ok = cudaSetDevice(dev) == cudaSuccess;
   const size_t piece = StagePool::kPiece;
   const size_t n_pieces = (bytes + piece - 1) / piece;
   size_t q = 0;
@@ -644,11 +685,64 @@ inline void stage_worker(int dev, const unsigned char* src, unsigned char* dst, 
     ok = cudaMemcpyAsync(dst + off, buf[b], len, cudaMemcpyHostToDevice, st) == cudaSuccess &&
          cudaEventRecord(ev[b], st) == cudaSuccess;
   }
-  if (st && cudaStreamSynchronize(st) != cudaSuccess) ok = false;
-  if (ev[0]) cudaEventDestroy(ev[0]);
-  if (ev[1]) cudaEventDestroy(ev[1]);
-  if (st) cudaStreamDestroy(st);
+  if (cudaStreamSynchronize(st) != cudaSuccess) ok = false;
   if (!ok) err->store(1);
+}
+
+// Device block (`lines` runs of `run` bytes, `src_pitch` apart) to pageable host memory (runs `dst_pitch` apart): the
+// driver stages such a copy through one thread that also takes the page faults of a result nobody has touched yet
+// (5 GB/s); here workers fetch pieces into their pinned buffers and move them on side by side.  The block must be
+// complete.  Returns KM_ENOMEM when there are no buffers to be had (nothing has been copied then).
+inline int stage_out(int dev, const unsigned char* src, size_t src_pitch, unsigned char* dst, size_t dst_pitch, size_t run,
+                     size_t lines) {
+  if (src_pitch == run && dst_pitch == run) { run *= lines; src_pitch = dst_pitch = run; lines = 1; }
+  StagePool& pool = StagePool::get();
+  std::lock_guard<std::mutex> lock(pool.busy);
+  const size_t piece = StagePool::kPiece;
+  const size_t per_line = (run + piece - 1) / piece, n_pieces = per_line * lines;
+  const int workers = (int)std::min<size_t>((size_t)stage_workers(1), n_pieces);
+  if (pool.ensure(2 * (size_t)workers) != KM_OK || !pool.ensure_lanes(dev, (size_t)workers)) return KM_ENOMEM;
+  std::vector<StagePool::Lane>& lanes = pool.lanes[dev];
+  std::atomic<int> err{0};
+  auto work = [&](int w) {
+    StagePool::Lane& lane = lanes[w];
+    void* buf[2] = {pool.bufs[2 * w], pool.bufs[2 * w + 1]};
+    bool ok = cudaSetDevice(dev) == cudaSuccess;
+    auto place = [&](size_t j, size_t* off_s, size_t* off_d, size_t* len) {
+      const size_t line = j / per_line, o = (j % per_line) * piece;
+      *off_s = line * src_pitch + o;
+      *off_d = line * dst_pitch + o;
+      *len = std::min(piece, run - o);
+    };
+    size_t os, od, len;
+    auto issue = [&](size_t j, int b) {
+      place(j, &os, &od, &len);
+      return cudaMemcpyAsync(buf[b], src + os, len, cudaMemcpyDeviceToHost, lane.st) == cudaSuccess &&
+             cudaEventRecord(lane.ev[b], lane.st) == cudaSuccess;
+    };
+    if (ok) ok = issue((size_t)w, 0);
+    int b = 0;
+    for (size_t j = (size_t)w; ok && j < n_pieces && err.load() == 0; j += workers, b ^= 1) {
+      if (j + workers < n_pieces) ok = issue(j + workers, b ^ 1);
+      ok = ok && cudaEventSynchronize(lane.ev[b]) == cudaSuccess;
+      if (!ok) break;
+      place(j, &os, &od, &len);
+      std::memcpy(dst + od, buf[b], len);
+    }
+    if (cudaStreamSynchronize(lane.st) != cudaSuccess) ok = false;
+    if (!ok) err.store(1);
+  };
+  std::vector<std::thread> threads;
+  int started = 1;
+  try {
+    for (; started < workers; ++started) threads.emplace_back(work, started);
+  } catch (const std::system_error&) {   // no more threads to be had: this one takes the other shares too
+  }
+  work(0);
+  for (int w = started; w < workers; ++w) work(w);
+  for (auto& t : threads) t.join();
+  if (err.load() != 0) { cudaGetLastError(); KM_FAIL(KM_ECUDA, "a staged copy to the host failed"); }
+  return KM_OK;
 }
 
 template <typename T>
@@ -675,15 +769,21 @@ int Engine<T>::upload_host_typed(const void* Xv, int src_dtype, size_t rows, siz
   const bool staged = stage_enabled && order == 'r' && rows * cols * esz >= ((size_t)64 << 20) &&
                       host_pointer_is_pageable(X);
   int workers_per_shard = 0;
+  std::vector<size_t> stage_lane0(g, 0);
   if (staged) {
-    // a single core copies far less than the bus carries (about 4 GB/s against 55 GB/s on the
-    // hosts measured), so nearly all of them are put to work
-    const unsigned hw = std::max(3u, std::thread::hardware_concurrency());
-    workers_per_shard = (int)std::max<size_t>(1, std::min<size_t>(14, hw - 2) / g);
+    workers_per_shard = stage_workers(g);
     StagePool& pool = StagePool::get();
     pool.busy.lock();
     upload_pool_locked = true;
-    if (pool.ensure(2 * workers_per_shard * g) != KM_OK) {
+    bool have = pool.ensure(2 * workers_per_shard * g) == KM_OK;
+    std::map<int, size_t> used;      // shards may share a device
+    for (size_t i = 0; have && i < g; ++i) {
+      DevGuard gd(shards[i].dev);
+      stage_lane0[i] = used[shards[i].dev];
+      used[shards[i].dev] += workers_per_shard;
+      have = pool.ensure_lanes(shards[i].dev, used[shards[i].dev]);
+    }
+    if (!have) {
       pool.busy.unlock();
       upload_pool_locked = false;
       workers_per_shard = 0;          // no pinned memory to be had: let the driver stage the copy
@@ -716,7 +816,8 @@ int Engine<T>::upload_host_typed(const void* Xv, int src_dtype, size_t rows, siz
       for (int w = 0; w < workers_per_shard; ++w) {
         const size_t b = 2 * (i * workers_per_shard + w);
         upload_threads.emplace_back(stage_worker, s.dev, X + off * cols * esz, dst, r * cols * esz, (size_t)w,
-                                    (size_t)workers_per_shard, pool.bufs[b], pool.bufs[b + 1], &upload_error);
+                                    (size_t)workers_per_shard, pool.bufs[b], pool.bufs[b + 1],
+                                    pool.lanes[s.dev][stage_lane0[i] + w], &upload_error);
       }
     } else if (order == 'r') {
       KM_CUDA(cudaMemcpyAsync(dst, X + off * cols * esz, r * cols * esz, cudaMemcpyHostToDevice, s.stream));

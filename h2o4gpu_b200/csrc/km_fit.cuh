@@ -551,6 +551,8 @@ int Engine<T>::transform_shard(int local, T* out_host, size_t ld) {
   cudaEventCreate(&e1);
   float ms_kernels = 0;
   int rc = KM_OK;
+  // below 16 MB the copy is over before the workers have started
+  const bool stage_result = host_pointer_is_pageable(out_host);
   bool wide = false, streamed = false;
   if constexpr (std::is_same<T, float>::value) {
     // tensor-core kernels with a store epilogue (they need max|x| for the operand scales, i.e. a checked
@@ -590,9 +592,20 @@ int Engine<T>::transform_shard(int local, T* out_host, size_t ld) {
     if (!wide && !streamed) rc = launch_tiles(s, s.X + r * (size_t)d, nr, nullptr, MODE_TRANSFORM, buf, batch, false);
     if (rc != KM_OK) break;
     cudaEventRecord(e1, s.stream);
-    cudaError_t ce = cudaMemcpy2DAsync(out_host + r, ld * sizeof(T), buf, batch * sizeof(T), nr * sizeof(T), k,
-                                       cudaMemcpyDeviceToHost, s.stream);
-    if (ce == cudaSuccess) ce = cudaStreamSynchronize(s.stream);
+    cudaError_t ce = cudaSuccess;
+    int staged = KM_ENOMEM;
+    if (stage_result && nr * (size_t)k * sizeof(T) >= ((size_t)16 << 20)) {
+      ce = cudaStreamSynchronize(s.stream);
+      if (ce == cudaSuccess)
+        staged = stage_out(s.dev, reinterpret_cast<const unsigned char*>(buf), batch * sizeof(T),
+                           reinterpret_cast<unsigned char*>(out_host + r), ld * sizeof(T), nr * sizeof(T), (size_t)k);
+      if (ce == cudaSuccess && staged != KM_OK && staged != KM_ENOMEM) { rc = staged; break; }
+    }
+    if (ce == cudaSuccess && staged != KM_OK) {
+      ce = cudaMemcpy2DAsync(out_host + r, ld * sizeof(T), buf, batch * sizeof(T), nr * sizeof(T), k,
+                             cudaMemcpyDeviceToHost, s.stream);
+      if (ce == cudaSuccess) ce = cudaStreamSynchronize(s.stream);
+    }
     if (ce != cudaSuccess) { set_error(std::string("transform copy: ") + cudaGetErrorString(ce)); rc = KM_ECUDA; }
     float ms = 0;
     if (cudaEventElapsedTime(&ms, e0, e1) == cudaSuccess) ms_kernels += ms;

@@ -391,6 +391,7 @@ extern "C" {
 const char* kmeans_last_error(void) { return km::g_err.c_str(); }
 int kmeans_trim_memory(void) {
   km::km_trim_pools();
+  km::StagePool::get().trim();
   return KM_OK;
 }
 int kmeans_last_fit_info(int* iterations, double* inertia) {

@@ -23,6 +23,9 @@ _sz = _c.c_size_t
 _vp = _c.c_void_p
 
 
+ENONFINITE = -6      # KM_ENONFINITE
+
+
 class KMeansLibError(RuntimeError):
     def __init__(self, code, msg):
         super().__init__("libh2o4gpu_kmeans: error %d: %s" % (code, msg))

@@ -1421,3 +1421,43 @@ def test_one_product_kernel_with_a_cluster_that_stays_empty(eng):
         h.fit(C, 2)
         assert _nearest_gap(X, h.centroids(), h.labels()) == 0
         h.close()
+
+
+# ---- host arrays: the data check and the way of a large result ---------------------------------
+@pytest.mark.parametrize("dtype", [np.float16, np.float32, np.float64])
+@pytest.mark.parametrize("bad", [np.nan, np.inf, -np.inf])
+def test_estimator_refuses_non_finite_data(built_lib, dtype, bad):
+    """fit (plain, weighted, given start) and predict report NaN / Inf in X as the wrapper always did, wherever in the
+    matrix it stands; integers pass."""
+    from h2o4gpu_b200 import KMeansH2O
+    rng = np.random.default_rng(3)
+    X = rng.standard_normal((2000, 9)).astype(dtype)
+    m = KMeansH2O(n_clusters=3, max_iter=3, random_state=1).fit(X)
+    Y = X.copy()
+    Y[1999, 8] = bad
+    for call in (lambda: KMeansH2O(n_clusters=3, random_state=1).fit(Y), lambda: m.predict(Y),
+                 lambda: KMeansH2O(n_clusters=3, random_state=1).fit(Y, sample_weight=np.ones(2000)),
+                 lambda: KMeansH2O(n_clusters=3, init="random", random_state=1).fit(Y),
+                 lambda: KMeansH2O(n_clusters=3, init=np.asarray(X[:3], np.float64)).fit(Y)):
+        with pytest.raises(ValueError, match="contains Inf or NaN"):
+            call()
+    assert m.predict(X).shape == (2000,)
+    KMeansH2O(n_clusters=3, max_iter=2, random_state=1).fit(rng.integers(0, 9, (500, 4)))
+
+
+@pytest.mark.parametrize("dtype,n,d,k", [(np.float32, 300_001, 5, 17), (np.float64, 700_000, 3, 9), (np.float32, 1000, 4, 3)])
+@pytest.mark.parametrize("batch", ["0", "131072"])
+def test_transform_result_reaches_the_host_whole(built_lib, monkeypatch, dtype, n, d, k, batch):
+    """Results above and below the size from which worker threads bring them down, in one block and in several whose
+    columns are not contiguous in the result, ragged last pieces: every distance equals numpy's."""
+    from h2o4gpu_b200 import KMeansH2O
+    monkeypatch.setenv("H2O4GPU_KM_TRANSFORM_BATCH_ROWS", batch)
+    rng = np.random.default_rng(n)
+    X = rng.standard_normal((n, d)).astype(dtype)
+    m = KMeansH2O(n_clusters=k)
+    m.cluster_centers_ = rng.standard_normal((k, d)).astype(dtype)
+    got = m.transform(X)
+    assert got.shape == (n, k)
+    for j in range(k):
+        want = ((X.astype(np.float64) - m.cluster_centers_[j].astype(np.float64)) ** 2).sum(1)
+        assert np.abs(got[:, j] - want).max() < (1e-4 if dtype == np.float32 else 1e-12) * want.max()
