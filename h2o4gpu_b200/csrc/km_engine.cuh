@@ -27,6 +27,7 @@
 #include "km_assign_dmma.cuh"
 #include "km_common.cuh"
 #include "km_finalize.cuh"
+#include "km_narrow.cuh"
 #include "km_nccl.h"
 #include "km_push.cuh"
 #include "km_refine.cuh"
@@ -1143,6 +1144,12 @@ int Engine<T>::launch_tiles(Shard<T>& s, const T* Xp, size_t nrows, int* labels,
                             size_t ld_out, bool count_changes, const IterState* gate) {
   bool vec = (d % VecOf<T>::N == 0) && ((reinterpret_cast<uintptr_t>(Xp) & 15) == 0);
   ++launches;
+  // narrow rows: the tile kernel pads them to 16 columns.  The float64 matrix unit does so too, but is still ahead from
+  // six columns (0.87 ps per score against (d + 2) 0.123) where it applies: more than 32 centroids, an even width.
+  if (mode == MODE_ASSIGN && narrow_shape_ok(k, d) &&
+      !(std::is_same<T, double>::value && d >= 6 && vec && dmma::shape_ok(k, d)))
+    return narrow_launch<T>(Xp, nrows, d, s.C[cur], k, s.cnorm, labels, count_changes ? s.st : nullptr, gate, s.num_sms,
+                            s.stream);
   return TileCfg<T>::go(Xp, nrows, d, s.C[cur], k, s.cnorm, labels, count_changes ? s.st : nullptr, out, ld_out,
                         mode, vec, s.stream, gate);
 }

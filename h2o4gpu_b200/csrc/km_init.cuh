@@ -78,6 +78,26 @@ mincost_update_kernel(const T* __restrict__ X, size_t n, int d, const int* __res
   }
 }
 
+// The same for at most eight columns, a row per thread (a warp per row left 29 of 32 lanes idle at three columns:
+// 35 us for 273,280 rows); the squares are added in the order of the warp's reduction, so the costs are the same bits.
+template <typename T>
+__global__ void __launch_bounds__(256)
+mincost_update_narrow_kernel(const T* __restrict__ X, size_t n, int d, const int* __restrict__ labels,
+                             const T* __restrict__ C, double* __restrict__ cost) {
+  for (size_t row = (size_t)blockIdx.x * 256 + threadIdx.x; row < n; row += (size_t)gridDim.x * 256) {
+    const T* x = X + row * (size_t)d;
+    const T* c = C + (size_t)labels[row] * d;
+    double q[8];
+#pragma unroll
+    for (int t = 0; t < 8; ++t) {
+      q[t] = 0;
+      if (t < d) { const double v = (double)x[t] - (double)c[t]; q[t] = v * v; }
+    }
+    const double s = ((q[0] + q[4]) + (q[2] + q[6])) + ((q[1] + q[5]) + (q[3] + q[7]));
+    cost[row] = fmin(cost[row], s);
+  }
+}
+
 // Bernoulli draw per row: selected when 2 k cost / phi exceeds the row's uniform number
 // (cost = weight * squared distance when sample weights are set).
 template <typename T>
@@ -369,7 +389,10 @@ int init_centroids(Engine<T>& e, int k, int seed, int method, std::vector<T>* ou
       if (rc != KM_OK) break;
       for (auto& s : e.shards) {
         DevGuard g(s.dev);
-        mincost_update_kernel<T><<<s.num_sms * 8, 256, 0, s.stream>>>(s.X, s.rows, d, s.labels, s.C[e.cur], s.dist);
+        if (d <= 8)
+          mincost_update_narrow_kernel<T><<<s.num_sms * 8, 256, 0, s.stream>>>(s.X, s.rows, d, s.labels, s.C[e.cur], s.dist);
+        else
+          mincost_update_kernel<T><<<s.num_sms * 8, 256, 0, s.stream>>>(s.X, s.rows, d, s.labels, s.C[e.cur], s.dist);
       }
     }
     double phi = 0;

@@ -1485,3 +1485,33 @@ def test_many_empty_clusters_are_repaired_like_the_oracle(eng, dtype, n_empty, c
     assert check_labels(X, C.astype(np.float64), got[1], labn) == 0
     assert len(moved) >= n_empty and got[2]["relocations"] == len(moved)
     assert rel_err(got[0], Cn) < (F32_TOL if dtype == np.float32 else F64_TOL)
+
+
+# ---- narrow rows ---------------------------------------------------------------------------------
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("n,d,k", [(1, 3, 17), (257, 1, 17), (5000, 2, 100), (200_001, 3, 64), (40_000, 4, 33),
+                                   (3000, 5, 1025), (1025, 6, 31), (9000, 7, 2049), (700_000, 8, 20)])
+def test_narrow_rows_labels(eng, dtype, n, d, k):
+    """Rows of at most eight columns and more than 16 centroids: one row and several rows per thread, one piece of
+    the table and several.  Labels are the float64 argmin but for near ties (float32 scores carry an error of up to
+    (d + 2) 2^-24 (|x|^2 + |c|^2), float64 ones 2^-53 of it), the lowest of equal centroids."""
+    rng = np.random.default_rng(n + d + k)
+    X = rng.uniform(-4, 4, (n, d)).astype(dtype)
+    C = rng.uniform(-4, 4, (k, d)).astype(dtype)
+    C[k // 2] = C[k // 3]
+    h = eng.ResidentKMeans(dtype=dtype)
+    h.upload(X)
+    h.set_centroids(C)
+    h.assign()
+    lab = h.labels()
+    h.close()
+    eps = 2.0 ** (-24 if dtype == np.float32 else -53)
+    Cd = C.astype(np.float64)
+    for s in range(0, n, 20_000):
+        x = X[s:s + 20_000].astype(np.float64)
+        dist = ((x[:, None, :] - Cd[None]) ** 2).sum(2) if k * x.shape[0] < 3e7 else \
+            (x * x).sum(1)[:, None] + (Cd * Cd).sum(1)[None] - 2 * x @ Cd.T
+        got = dist[np.arange(x.shape[0]), lab[s:s + 20_000]]
+        bound = 2 * (d + 2) * eps * ((x * x).sum(1) + (Cd * Cd).sum(1).max()) + 1e-12
+        assert (got - dist.min(1) <= bound).all()
+    assert not (lab == max(k // 2, k // 3)).any()      # the copy has the higher index
