@@ -1196,7 +1196,7 @@ int Engine<T>::launch_smallk(Shard<T>& s, bool update, T scale) {
   size_t rpc = (s.rows + target - 1) / target;
   // A CTA takes 64 rows a step; the fused update ends with a drain of k d sums into global memory, which 8 k rows
   // outweigh.  With 512 rows at least, 100,000 x 32 rows were 196 CTAs of eight dependent steps each and took 56 us,
-  // 2,000 rows 34 us in four CTAs; with 64 it is 54 and 10 us.
+  // 2,000 rows 34 us in four CTAs; with 64 the latter take 10 us (4 since the exchanges overlap, km_smallk.cuh).
   rpc = std::max<size_t>(rpc, update ? std::max<size_t>(64, 8 * (size_t)k) : 64);
   rpc = std::min<size_t>(rpc, kFlushRows);
   size_t grid = (s.rows + rpc - 1) / rpc;
