@@ -288,7 +288,18 @@ struct Engine : EngineBase {
   int stream_refresh(Shard<T>& s);   // operand table and plan of the streaming kernel for the current centroids
   int tc_refresh(Shard<T>& s);  // split the current centroids for the tensor-core kernel
   int launch_assign(Shard<T>& s, bool use_tc, bool count_changes);
-  bool tc_split_build = false;   // the running fit has enough iterations to pay for the split copy of X
+  tc::SplitBuild tc_split_build = tc::SplitBuild::no;   // whether the running fit pays for the split copy of X
+  // Begins a call that labels rows.  The caller may have written other values into a matrix it lends
+  // (attach_device) since the last call, so the rounded rows are made from what is there now: they live as long as one
+  // call.  Only the split copy of a long fit stays, as it always did, and what was taken when the matrix was
+  // attached (max |x|, row norms, padded rows).  A matrix this handle uploaded cannot change under it.
+  void drop_row_copies() {
+    for (auto& s : shards) {
+      if (s.X == s.X_owned) continue;
+      s.tchp.of = nullptr;
+      if (!s.tcp.xsplit_kept) s.tcp.xsplit_of = nullptr;
+    }
+  }
   float tc_sx = 1.f, tc_sb = 1.f;   // operand scales of the tensor-core kernel
   double cbound = 0;                // bound on |centroid coordinate|: max(|x|, |initial centroids|)
 
@@ -473,6 +484,7 @@ int Engine<T>::attach_device(int local, const T* dX, size_t rows, size_t cols, s
   // even when the new one has the same address and shape
   s.tcp.xnorm_of = nullptr;
   s.tcp.xsplit_of = nullptr;
+  s.tcp.xsplit_kept = false;
   s.tcp.ready = false;
   s.tcbp.ready = false;
   s.tchp.of = nullptr;

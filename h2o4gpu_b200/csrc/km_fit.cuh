@@ -170,6 +170,7 @@ int Engine<T>::fit(int k_, int max_iter, double threshold, const T* init, int fl
   const double t_start = now_s();
   launches = 0;
   KM_TRY(check_data());
+  drop_row_copies();
   KM_TRY(set_centroids(k_, init));
 
   // fixed-point scale from the global max |x|: xmax < 2^e, first piece <= 2^15 (with sample
@@ -190,8 +191,10 @@ int Engine<T>::fit(int k_, int max_iter, double threshold, const T* init, int fl
   const bool use_tc = !fused && tc_ok(flags);
   // the fp16 copy of X (d = 64 tensor-core kernel without converter warps) takes the place of the row norms'
   // pass and costs about as much more as one iteration saves
-  tc_split_build = max_iter >= 3 || (flags & KM_FIT_PRESPLIT);
-  struct SplitBuildGuard { bool& f; ~SplitBuildGuard() { f = false; } } split_build_guard{tc_split_build};
+  tc_split_build = (max_iter >= 16 || (flags & KM_FIT_PRESPLIT)) ? tc::SplitBuild::keep
+                   : max_iter >= 3                               ? tc::SplitBuild::call
+                                                                 : tc::SplitBuild::no;
+  struct SplitBuildGuard { tc::SplitBuild& f; ~SplitBuildGuard() { f = tc::SplitBuild::no; } } split_build_guard{tc_split_build};
   // incremental M-step (km_accumulate_delta.cuh): on unless the caller or the environment asks
   // for a full recomputation every iteration; a shard switches to it, on the device, in the
   // iterations where at most 1/8 of its labels moved (kDeltaFraction)

@@ -342,6 +342,7 @@ int init_centroids(Engine<T>& e, int k, int seed, int method, std::vector<T>* ou
   if (seed < 0) seed = (int)(std::random_device{}() & 0x7fffffff);
   const unsigned long long useed = (unsigned long long)(unsigned int)seed;
   KM_TRY(e.check_data());
+  e.drop_row_copies();
 
   // 1. first candidate
   unsigned int c4[4] = {0u, 0u, 0u, kStreamFirst};

@@ -63,6 +63,7 @@ struct Plan {
   const float* xsplit_of = nullptr;
   size_t xsplit_rows = 0;
   float xsplit_sx = 0.f;
+  bool xsplit_kept = false;     // made by a long fit (or on request): good until other data is attached
   bool xsplit_failed = false;   // no memory for it: stay with the converting kernel
   CUtensorMap tmXh;
 
@@ -113,6 +114,7 @@ inline int ensure_xnorm(Plan& pl, const float* X, size_t rows, int d, int num_sm
 
 // The fp16 copy of X for the kernel variant without converter warps (d = 64): made when the
 // matrix, its size or the scale changed; costs one pass over X and half as much memory again.
+enum class SplitBuild { no, call, keep };   // not at all, for the running call, until other data is attached
 inline bool presplit_enabled() {
   static const bool on = [] {
     const char* e = std::getenv("H2O4GPU_KM_TC_PRESPLIT");
@@ -121,10 +123,13 @@ inline bool presplit_enabled() {
   return on;
 }
 inline bool ensure_xsplit(Plan& pl, const float* X, size_t rows, int d, float sx, int num_sms, cudaStream_t stream,
-                          bool allow_build) {
+                          SplitBuild build) {
   if (d != 64 || !presplit_enabled() || pl.xsplit_failed) return false;
-  if (pl.xsplit && pl.xsplit_of == X && pl.xsplit_rows == rows && pl.xsplit_sx == sx) return true;
-  if (!allow_build) return false;   // a single pass (predict) does not pay for the split
+  if (pl.xsplit && pl.xsplit_of == X && pl.xsplit_rows == rows && pl.xsplit_sx == sx) {
+    pl.xsplit_kept = pl.xsplit_kept || build == SplitBuild::keep;
+    return true;
+  }
+  if (build == SplitBuild::no) return false;   // a single pass (predict) does not pay for the split
   if (pl.xsplit_cap < rows) {
     km_free(pl.xsplit);
     km_free(pl.xrowq);
@@ -147,6 +152,7 @@ inline bool ensure_xsplit(Plan& pl, const float* X, size_t rows, int d, float sx
   pl.xsplit_of = X;
   pl.xsplit_rows = rows;
   pl.xsplit_sx = sx;
+  pl.xsplit_kept = build == SplitBuild::keep;
   return true;
 }
 
@@ -212,12 +218,12 @@ inline float tol_floor_of(int d) { return 1.1920928955078125e-07f * std::sqrt((f
 
 inline int launch(Plan& pl, int* labels, IterState* st, bool count_changes, unsigned int* amb_rows,
                   unsigned int* amb_seg, float tol_rel, int num_sms, cudaStream_t stream, unsigned int* moved_bits,
-                  uint4* amb_near, bool allow_split_build, int* launches) {
+                  uint4* amb_near, SplitBuild split_build, int* launches) {
   const size_t tiles = (pl.x_rows + kBM - 1) / kBM;
   if (tiles > 0x7fffffffULL / kBM) KM_FAIL(KM_EINVAL, "shard too large for the tensor-core kernel");
   const int grid = (int)std::min<size_t>(tiles, (size_t)num_sms);
   const unsigned int seg_cap = (unsigned int)amb_seg_rows(pl.x_rows, num_sms);
-  const bool pre = ensure_xsplit(pl, pl.x_base, pl.x_rows, pl.d, pl.sx, num_sms, stream, allow_split_build);
+  const bool pre = ensure_xsplit(pl, pl.x_base, pl.x_rows, pl.d, pl.sx, num_sms, stream, split_build);
   if (!pre) KM_TRY(ensure_xnorm(pl, pl.x_base, pl.x_rows, pl.d, num_sms, stream));
   auto go = [&](auto fn, const CUtensorMap& tmX, bool p) {
     fn<<<grid, kThreads, smem_bytes(pl.d, pl.npad, p), stream>>>(

@@ -310,6 +310,7 @@ template <typename T>
 static int assign_sync(km::Engine<T>* e) {
   KM_TRY(e->check_data());
   if (e->shards.empty()) KM_FAIL(KM_ESTATE, "no data attached to the handle");
+  e->drop_row_copies();
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   {
     km::DevGuard g(e->shards[0].dev);

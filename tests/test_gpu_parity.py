@@ -1515,3 +1515,39 @@ def test_narrow_rows_labels(eng, dtype, n, d, k):
         bound = 2 * (d + 2) * eps * ((x * x).sum(1) + (Cd * Cd).sum(1).max()) + 1e-12
         assert (got - dist.min(1) <= bound).all()
     assert not (lab == max(k // 2, k // 3)).any()      # the copy has the higher index
+
+
+# ---- a lent matrix that changes between calls ------------------------------------------------------
+@pytest.mark.parametrize("dtype,n,d,k,iters", [(np.float64, 30_000, 40, 100, 3), (np.float32, 130_001, 64, 260, 3),
+                                               (np.float32, 60_000, 50, 200, 2), (np.float32, 50_000, 64, 100, 5)])
+def test_values_written_into_an_attached_matrix_are_seen(eng, dtype, n, d, k, iters):
+    """Fit, other values into the same device buffer (the same rows in another order, so that max |x| holds), fit and
+    assign without attaching again: what a fresh handle on the new values gives."""
+    import torch
+    rng = np.random.default_rng(d * k)
+    centers = rng.uniform(-6, 6, (k, d))
+    a = (centers[rng.integers(0, k, n)] + rng.standard_normal((n, d))).astype(dtype)
+    C = a[rng.choice(n, k, replace=False)].copy()
+    X = torch.as_tensor(a, device="cuda")
+    h = eng.ResidentKMeans(dtype=dtype)
+    h.attach_device(0, X.data_ptr(), n, d)
+    h.fit(C, iters)
+    assert h.stats()["path"] == 3
+    X.copy_(torch.as_tensor(a[::-1].copy(), device="cuda"))
+    torch.cuda.synchronize()
+    h.fit(C, iters)
+    got = h.centroids(), h.labels()
+    fresh = eng.ResidentKMeans(dtype=dtype)
+    fresh.attach_device(0, X.data_ptr(), n, d)
+    fresh.fit(C, iters)
+    assert np.array_equal(got[0], fresh.centroids()) and np.array_equal(got[1], fresh.labels())
+    X.copy_(torch.as_tensor(a, device="cuda"))
+    torch.cuda.synchronize()
+    h.set_centroids(C)
+    h.assign()
+    fresh.attach_device(0, X.data_ptr(), n, d)
+    fresh.set_centroids(C)
+    fresh.assign()
+    assert np.array_equal(h.labels(), fresh.labels())
+    h.close()
+    fresh.close()
