@@ -5,6 +5,7 @@
 #include <cuda_fp16.h>
 #include <algorithm>
 #include <cstdlib>
+#include <map>
 #include <mutex>
 
 #include <cuda_runtime.h>
@@ -126,15 +127,33 @@ struct DevicePools {
   }
 };
 
+// A limit on what the calling thread may hold through km_malloc, so that a test can run a call out of device memory
+// on the host alone (kmeans_selftest_alloc_limit).  Off unless that has been called.
+struct AllocLimit {
+  bool on = false;
+  size_t left = 0;
+  std::map<void*, size_t> held;
+  static AllocLimit& get() {
+    static thread_local AllocLimit l;
+    return l;
+  }
+};
+
 inline cudaError_t km_malloc_bytes(void** p, size_t bytes) {
   int dev = 0;
   cudaError_t ce = cudaGetDevice(&dev);
   if (ce != cudaSuccess) return ce;
+  AllocLimit& lim = AllocLimit::get();
+  if (lim.on && bytes > lim.left) return cudaErrorMemoryAllocation;
   DevicePools& dp = DevicePools::get();
-  if (dp.mode(dev) != 1) return cudaMalloc(p, bytes);
-  ce = cudaMallocFromPoolAsync(p, std::max<size_t>(bytes, 1), dp.pool[dev], dp.stream[dev]);
-  if (ce != cudaSuccess) return ce;
-  return cudaStreamSynchronize(dp.stream[dev]);
+  if (dp.mode(dev) != 1) {
+    ce = cudaMalloc(p, bytes);
+  } else {
+    ce = cudaMallocFromPoolAsync(p, std::max<size_t>(bytes, 1), dp.pool[dev], dp.stream[dev]);
+    if (ce == cudaSuccess) ce = cudaStreamSynchronize(dp.stream[dev]);
+  }
+  if (lim.on && ce == cudaSuccess) { lim.left -= bytes; lim.held[*p] = bytes; }
+  return ce;
 }
 template <typename P>
 inline cudaError_t km_malloc(P** p, size_t bytes) { return km_malloc_bytes(reinterpret_cast<void**>(p), bytes); }
@@ -144,11 +163,36 @@ inline cudaError_t km_free(void* p) {
   int dev = 0;
   cudaError_t ce = cudaGetDevice(&dev);
   if (ce != cudaSuccess) return ce;
+  AllocLimit& lim = AllocLimit::get();
+  if (lim.on) {
+    auto it = lim.held.find(p);
+    if (it != lim.held.end()) { lim.left += it->second; lim.held.erase(it); }
+  }
   DevicePools& dp = DevicePools::get();
   if (dp.mode(dev) != 1) return cudaFree(p);
   ce = cudaDeviceSynchronize();      // nothing in flight may still use the buffer
   if (ce != cudaSuccess) return ce;
   return cudaFreeAsync(p, dp.stream[dev]);
+}
+
+// Whether to take `bytes` for a copy that a call can do without (rounded rows): as much again and 1 GB have to stay
+// free, for what this handle and its user allocate later.  Below 256 MB the question costs more than it guards.
+inline bool km_room_for(size_t bytes) {
+  if (bytes < ((size_t)256 << 20)) return true;
+  size_t free_b = 0, total_b = 0;
+  int dev = 0;
+  if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || cudaGetDevice(&dev) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  DevicePools& dp = DevicePools::get();
+  if (dp.mode(dev) == 1) {   // what the pool holds and nobody uses is free too
+    unsigned long long held = 0, used = 0;
+    if (cudaMemPoolGetAttribute(dp.pool[dev], cudaMemPoolAttrReservedMemCurrent, &held) == cudaSuccess &&
+        cudaMemPoolGetAttribute(dp.pool[dev], cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess && held > used)
+      free_b += held - used;
+  }
+  return free_b >= 2 * bytes + ((size_t)1 << 30);
 }
 
 inline void km_trim_pools() {

@@ -1377,8 +1377,13 @@ int Engine<T>::tc_refresh(Shard<T>& s) {
     if (s.rows > 0xffffffffULL) KM_FAIL(KM_EINVAL, "shard too large for the tensor-core kernel");
     KM_TRY(ensure_amb(s, tc_kind() == 1));
     const int kind = tc_kind();
-    if (half) s.tchp.on = tch::half_rows<T>(s.tchp, s.X, s.rows, d, tc_sx, s.num_sms, s.stream, &launches);
-    if (d % 4 != 0) KM_TRY(ensure_xpad(s, !s.tchp.on));
+    // what the call cannot do without comes before the rounded rows: tc_ok() has seen that it fits
+    if (d % 4 != 0) KM_TRY(ensure_xpad(s, !half));
+    if (half) {
+      KM_TRY(tcb::big_tables(s.tcbp, k, d, true));
+      s.tchp.on = tch::half_rows<T>(s.tchp, s.X, s.rows, d, tc_sx, s.num_sms, s.stream, &launches);
+      if (!s.tchp.on && d % 4 != 0) KM_TRY(ensure_xpad(s));
+    }
     if (kind == 3) {
       KM_TRY(tc::ensure_xnorm(s.tcp, xtc(s), s.rows, dtc(), s.num_sms, s.stream));   // float4 loads: the aligned rows
       KM_TRY(tcw::wide_setup(s.tcwp, xtc(s), s.rows, k, d, dtc()));

@@ -136,9 +136,13 @@ inline bool ensure_xsplit(Plan& pl, const float* X, size_t rows, int d, float sx
     pl.xsplit = nullptr;
     pl.xrowq = nullptr;
     pl.xsplit_cap = 0;
-    if (km_malloc(&pl.xsplit, rows * 64 * sizeof(__half)) != cudaSuccess ||
+    const size_t row_bytes = 64 * sizeof(__half) + sizeof(float2);
+    if (!km_room_for(rows * row_bytes) || km_malloc(&pl.xsplit, rows * 64 * sizeof(__half)) != cudaSuccess ||
         km_malloc(&pl.xrowq, rows * sizeof(float2)) != cudaSuccess) {
       cudaGetLastError();
+      km_free(pl.xsplit);   // one without the other is of no use
+      pl.xsplit = nullptr;
+      pl.xrowq = nullptr;
       pl.xsplit_failed = true;
       return false;
     }
@@ -394,22 +398,27 @@ inline bool half_grow(P** p, size_t* cap, size_t need) {
 }
 
 // Rounded rows of X (made when the matrix or the scale changed) and the candidate list.  False: no memory for
-// them, the caller stays with the kernels that read the rows as they are.
+// them (none of it is held then), the caller stays with the kernels that read the rows as they are.
 template <typename T>
 inline bool half_rows(HalfPlan& pl, const T* X, size_t rows, int d, float sx, int num_sms, cudaStream_t stream,
                       int* launches) {
   const int ldh = (d + 7) / 8 * 8;
   // a quarter of the rows: settling an open row costs about twice its share of the pass that needs no list
   const size_t cap = std::max<size_t>(rows / 4, std::min<size_t>(rows, 4096));
-  if (pl.cand_cap < cap) {
+  const size_t elems = rows * (size_t)ldh;
+  if (pl.cand_cap < cap || pl.xh_cap < elems || pl.rowq_cap < rows) {
     size_t have = pl.cand_cap;
-    pl.cand_cap = 0;
-    if (!half_grow(&pl.cand_near, &have, cap)) return false;
-    pl.cand_cap = (unsigned int)cap;
+    pl.of = nullptr;
+    if (!km_room_for(elems * sizeof(__half) + rows * sizeof(float2) + cap * sizeof(uint4)) ||
+        !half_grow(&pl.cand_near, &have, cap) || !half_grow(&pl.xh, &pl.xh_cap, elems) ||
+        !half_grow(&pl.rowq, &pl.rowq_cap, rows)) {
+      pl.release();
+      return false;
+    }
+    pl.cand_cap = (unsigned int)have;
   }
   if (pl.of == X && pl.rows == rows && pl.sx == sx && pl.ldh == ldh) return true;
   pl.of = nullptr;
-  if (!half_grow(&pl.xh, &pl.xh_cap, rows * (size_t)ldh) || !half_grow(&pl.rowq, &pl.rowq_cap, rows)) return false;
   int lpr = 1;
   while (lpr < 32 && lpr * 4 < ldh) lpr *= 2;
   if (d % 4 == 0 && (reinterpret_cast<uintptr_t>(X) & 15) == 0)

@@ -411,6 +411,14 @@ int kmeans_set_wait_limits(double peer_wait_ms, double mbarrier_wait_ms) {
   return KM_OK;
 }
 
+int kmeans_selftest_alloc_limit(long long bytes) {
+  km::AllocLimit& l = km::AllocLimit::get();
+  l.on = bytes >= 0;
+  l.left = bytes >= 0 ? (size_t)bytes : 0;
+  l.held.clear();
+  return KM_OK;
+}
+
 int kmeans_selftest_wait_timeout(int gpu_id, int which, int* device_code) {
   int visible = 0;
   if (cudaGetDeviceCount(&visible) != cudaSuccess || gpu_id < 0 || gpu_id >= visible)

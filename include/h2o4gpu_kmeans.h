@@ -61,6 +61,11 @@ int kmeans_set_wait_limits(double peer_wait_ms, double mbarrier_wait_ms);
  * the device usable.  Set short limits first. */
 int kmeans_selftest_wait_timeout(int gpu_id, int which, int* device_code);
 
+/* From now on the calling thread's device allocations inside the library fail once they would hold more than
+ * `bytes` beyond what is held now (negative: no limit), as if the device were full: for tests of what a call
+ * does without in that case.  Nothing is asked of the device. */
+int kmeans_selftest_alloc_limit(long long bytes);
+
 /* ---- 1. the reference's entry points ------------------------------------ */
 
 /* Fit (dopredict == 0) or predict (dopredict == 1).

@@ -1551,3 +1551,45 @@ def test_values_written_into_an_attached_matrix_are_seen(eng, dtype, n, d, k, it
     assert np.array_equal(h.labels(), fresh.labels())
     h.close()
     fresh.close()
+
+
+# ---- device memory that runs short ------------------------------------------------------------------
+@pytest.mark.parametrize("dtype,d,k", [(np.float32, 50, 64), (np.float32, 64, 260), (np.float32, 64, 100),
+                                       (np.float64, 40, 100)])
+def test_a_fit_that_fits_without_the_rounded_rows_runs(eng, built_lib, dtype, d, k):
+    """Device memory limited to what a fit needs when it reads the rows as they are (labels, distances, lists of rows,
+    norms, and for rows that are not 16-byte aligned the padded copy) and in small steps from there on to beyond what the
+    rounded rows take: every fit runs, with the same result.  The limit counts allocations on the host."""
+    import torch
+    from h2o4gpu_b200.libs import lib_kmeans
+    lib = lib_kmeans.cdll()
+    rng = np.random.default_rng(d + k)
+    n, mb = 400_000, 1 << 20
+    centers = rng.uniform(-6, 6, (k, d))
+    a = (centers[rng.integers(0, k, n)] + rng.standard_normal((n, d))).astype(dtype)
+    C = a[rng.choice(n, k, replace=False)].copy()
+    X = torch.as_tensor(a, device="cuda")
+
+    def fit(limit):
+        h = eng.ResidentKMeans(dtype=dtype)
+        h.attach_device(0, X.data_ptr(), n, d)
+        lib.kmeans_selftest_alloc_limit(limit)
+        try:
+            h.fit(C, 3)
+        finally:
+            lib.kmeans_selftest_alloc_limit(-1)
+        out = h.centroids(), h.labels()
+        h.close()
+        return out
+
+    want = fit(-1)
+    per_row = 8 + 4 + 4 + 4 + 1          # distances, previous labels, list of rows, norms, moved rows (a bit each)
+    if (d, k) == (64, 100):
+        per_row += 16                    # candidates of a listed row
+    if d % 4:
+        per_row += 4 * ((d + 3) // 4 * 4)
+    for extra in range(24, 24 + 96):     # 24 MB: tables of the centroids and sums
+        got = fit(n * per_row + extra * mb)
+        assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1]), extra
+    with pytest.raises(lib_kmeans.KMeansLibError):
+        fit(n * 8)
