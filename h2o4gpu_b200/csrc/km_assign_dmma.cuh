@@ -186,8 +186,7 @@ assign_kernel(const double* __restrict__ X, size_t n, int d, const double* __res
 
 inline int launch(const double* X, size_t n, int d, const double* C, int k, const double* cnorm, int* labels,
                   IterState* st, cudaStream_t stream, const IterState* gate) {
-  // per device, so set on every launch (cheap)
-  KM_CUDA(cudaFuncSetAttribute(assign_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes));
+  KM_CUDA(allow_smem(assign_kernel, kSmemBytes));
   // without this the driver sizes the shared-memory carve-out for one CTA and only one is resident
   cudaFuncSetAttribute(assign_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
   const size_t grid = (n + BM - 1) / BM;

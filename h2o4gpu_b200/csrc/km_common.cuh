@@ -7,6 +7,7 @@
 #include <cstdlib>
 #include <map>
 #include <mutex>
+#include <utility>
 
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -203,6 +204,27 @@ inline void km_trim_pools() {
       cudaStreamSynchronize(dp.stream[dev]);
       cudaMemPoolTrimTo(dp.pool[dev], 0);
     }
+}
+
+// Lets `fn` ask for `bytes` of dynamic shared memory.  The limit belongs to the kernel on a device, for every handle and
+// thread of the process, so it is only ever raised: set to what the launch at hand needs, a handle with few centroids
+// would lower it under another one's launch.
+inline cudaError_t allow_smem(const void* fn, size_t bytes) {
+  static std::mutex m;
+  static std::map<std::pair<int, const void*>, size_t> limit;
+  int dev = 0;
+  cudaError_t ce = cudaGetDevice(&dev);
+  if (ce != cudaSuccess) return ce;
+  std::lock_guard<std::mutex> lock(m);
+  size_t& l = limit[{dev, fn}];
+  if (bytes <= l) return cudaSuccess;
+  ce = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  if (ce == cudaSuccess) l = bytes;
+  return ce;
+}
+template <typename R, typename... A>
+inline cudaError_t allow_smem(R (*fn)(A...), size_t bytes) {
+  return allow_smem(reinterpret_cast<const void*>(fn), bytes);
 }
 
 // ---- fixed-point centroid sums ------------------------------------------------

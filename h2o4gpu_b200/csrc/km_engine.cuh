@@ -321,7 +321,7 @@ struct Engine : EngineBase {
     const size_t table_bytes = (size_t)k * d * sizeof(double);
     if (vec_ok(s) && table_bytes <= (size_t)96 * 1024) {
       // small tables: gather from a copy in shared memory, as many CTAs per SM as fit beside it
-      cudaFuncSetAttribute(rowdist_kernel<T, V, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
+      allow_smem(rowdist_kernel<T, V, true>, 96 * 1024);
       int per_sm = (int)((size_t)200 * 1024 / (table_bytes + 1024));
       per_sm = per_sm > 8 ? 8 : (per_sm < 1 ? 1 : per_sm);
       rowdist_kernel<T, V, true><<<s.num_sms * per_sm, 256, table_bytes, s.stream>>>(s.X, s.rows, d, s.labels, cd,
@@ -336,7 +336,7 @@ struct Engine : EngineBase {
     if constexpr (std::is_same<T, float>::value) {
       const size_t smem = (size_t)16 * d;
       if (smem > 48 * 1024)
-        KM_CUDA(cudaFuncSetAttribute(tcb::refine_big_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        KM_CUDA(allow_smem(tcb::refine_big_kernel, smem));
       tcb::refine_big_kernel<<<s.num_sms * 8, tcb::kRefineBigThreads, smem, s.stream>>>(
           s.X, d, s.Cd[cur], k, s.amb_rows, s.st, s.labels, count_changes ? 1 : 0);
       KM_CUDA(cudaGetLastError());
@@ -1216,7 +1216,7 @@ int Engine<T>::launch_smallk(Shard<T>& s, bool update, T scale) {
   if (vec) {
     auto fn = update ? smallk_pick<T, V, kSmallKRpw>(k, &K) : smallk_pick<T, V, kSmallKRpwAssign>(k, &K);
     smem = smallk_smem_bytes<T>(K, d, update);
-    e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    e = allow_smem(fn, smem);
     if (e != cudaSuccess) KM_CUDA(e);
     // without this the driver sizes the shared-memory carve-out for one CTA and only one is resident
     cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
@@ -1226,7 +1226,7 @@ int Engine<T>::launch_smallk(Shard<T>& s, bool update, T scale) {
   } else {
     auto fn = update ? smallk_pick<T, 1, kSmallKRpw>(k, &K) : smallk_pick<T, 1, kSmallKRpwAssign>(k, &K);
     smem = smallk_smem_bytes<T>(K, d, update);
-    e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    e = allow_smem(fn, smem);
     if (e != cudaSuccess) KM_CUDA(e);
     cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
     fn<<<(unsigned)grid, kSmallKThreads, smem, s.stream>>>(s.X, s.rows, d, s.C[cur], k, s.cnorm, s.labels, s.st,
@@ -1242,8 +1242,7 @@ template <int GS, int VPT>
 static int launch_sorted_gs(const float* X, size_t rows, int d, const int* labels, int k, long long* gs,
                             unsigned long long* gc, float scale30, const SortPlan& p, cudaStream_t stream,
                             const unsigned long long* gate, unsigned long long limit) {
-  KM_CUDA(cudaFuncSetAttribute(sorted_accumulate_kernel<GS, VPT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)p.smem_bytes));
+  KM_CUDA((allow_smem(sorted_accumulate_kernel<GS, VPT>, p.smem_bytes)));
   sorted_accumulate_kernel<GS, VPT><<<p.grid, kSortThreads, p.smem_bytes, stream>>>(
       X, rows, d, labels, k, gs, gc, scale30, p.tile_rows, p.smem_acc, gate, limit);
   KM_CUDA(cudaGetLastError());
@@ -1315,11 +1314,11 @@ int Engine<T>::launch_accumulate(Shard<T>& s, T scale, long long* dst, const uns
   if ((unsigned long long)rpp * dv * dv >= (1ULL << 40)) KM_FAIL(KM_EINVAL, "cols too large for the centroid-sum kernel");
   unsigned long long magic = fastdiv_magic((unsigned)dv);
   if (vec) {
-    KM_CUDA(cudaFuncSetAttribute(accumulate_kernel<T, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    KM_CUDA((allow_smem(accumulate_kernel<T, V>, smem)));
     accumulate_kernel<T, V><<<(unsigned)grid, kAccThreads, smem, s.stream>>>(
         s.X, s.rows, d, s.labels, k, kc, n_slices, gs, gc, scale, (unsigned)rpp, magic, gate, limit, W, (T)w_scale);
   } else {
-    KM_CUDA(cudaFuncSetAttribute(accumulate_kernel<T, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    KM_CUDA((allow_smem(accumulate_kernel<T, 1>, smem)));
     accumulate_kernel<T, 1><<<(unsigned)grid, kAccThreads, smem, s.stream>>>(
         s.X, s.rows, d, s.labels, k, kc, n_slices, gs, gc, scale, (unsigned)rpp, magic, gate, limit, W, (T)w_scale);
   }
@@ -1521,7 +1520,7 @@ int Engine<T>::launch_assign(Shard<T>& s, bool use_tc, bool count_changes) {
       const int grid = (int)std::min<size_t>(tiles, (size_t)s.num_sms);
       IterState* stp = count_changes ? s.st : nullptr;
       auto go = [&](auto fn) -> int {
-        KM_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        KM_CUDA(allow_smem(fn, smem));
         fn<<<grid, sks::kThreads, smem, s.stream>>>(s.X, s.rows, d, s.C[cur], k, s.cnorm, s.labels, stp);
         KM_CUDA(cudaGetLastError());
         ++launches;
@@ -1632,8 +1631,7 @@ int Engine<T>::launch_delta(Shard<T>& s, T scale, const unsigned long long* gate
   const T wsc = (T)w_scale;
   if (bitmap_env && !W && s.pflush && smem <= 100 * 1024 && s.moved_bits_valid && vec_ok(s)) {
     // the E-step left a map of the rows that moved: no label scan
-    KM_CUDA(cudaFuncSetAttribute(delta_accumulate_bitmap_kernel<T, V>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)smem));
+    KM_CUDA((allow_smem(delta_accumulate_bitmap_kernel<T, V>, smem)));
     delta_accumulate_bitmap_kernel<T, V><<<s.num_sms * 2, kDeltaThreads, smem, s.stream>>>(
         s.X, s.rows, d, s.labels, s.labels_prev, s.moved_bits, k, fs, fc, scale, gate, limit);
     KM_CUDA(cudaGetLastError());
@@ -1643,13 +1641,11 @@ int Engine<T>::launch_delta(Shard<T>& s, T scale, const unsigned long long* gate
   if (smem <= 200 * 1024 && s.pflush) {
     // centroid table small enough for shared accumulators: one or two CTAs per SM net their rows' moves
     if (vec_ok(s)) {
-      KM_CUDA(cudaFuncSetAttribute(delta_accumulate_smem_kernel<T, V>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)smem));
+      KM_CUDA((allow_smem(delta_accumulate_smem_kernel<T, V>, smem)));
       delta_accumulate_smem_kernel<T, V><<<s.num_sms * (smem <= 100 * 1024 ? 2 : 1), kDeltaThreads, smem, s.stream>>>(
           s.X, s.rows, d, s.labels, s.labels_prev, k, fs, fc, scale, gate, limit, W, wsc);
     } else {
-      KM_CUDA(cudaFuncSetAttribute(delta_accumulate_smem_kernel<T, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)smem));
+      KM_CUDA((allow_smem(delta_accumulate_smem_kernel<T, 1>, smem)));
       delta_accumulate_smem_kernel<T, 1><<<s.num_sms * (smem <= 100 * 1024 ? 2 : 1), kDeltaThreads, smem, s.stream>>>(
           s.X, s.rows, d, s.labels, s.labels_prev, k, fs, fc, scale, gate, limit, W, wsc);
     }

@@ -99,7 +99,7 @@ inline int narrow_launch_d(const T* X, size_t n, const T* C, int k, const T* cno
   auto go = [&](auto fn, int R) -> int {
     const size_t per = (size_t)kNarrowThreads * R, grid = (n + per - 1) / per;
     if (grid > 0x7fffffffULL) KM_FAIL(KM_EINVAL, "shard too large for one launch");
-    KM_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    KM_CUDA(allow_smem(fn, smem));
     fn<<<(unsigned)grid, kNarrowThreads, smem, stream>>>(X, n, C, k, cnorm, labels, st, gate);
     KM_CUDA(cudaGetLastError());
     return KM_OK;

@@ -175,15 +175,6 @@ inline int setup(Plan& pl, const float* X, size_t rows, int k, int d, int num_sm
   KM_TRY(make_map(&pl.tmX, X, rows, d, kBM, 4));
   KM_TRY(make_map(&pl.tmBhi, pl.bhi, npad, 64, npad, 2));
   KM_TRY(make_map(&pl.tmBlo, pl.blo, npad, 64, npad, 2));
-  if (d == 32) {
-    KM_CUDA(cudaFuncSetAttribute(assign_tc_kernel<32, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)smem_bytes(d, npad, false)));
-  } else {
-    KM_CUDA(cudaFuncSetAttribute(assign_tc_kernel<64, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)smem_bytes(d, npad, false)));
-    KM_CUDA(cudaFuncSetAttribute(assign_tc_kernel<64, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)smem_bytes(d, npad, true)));
-  }
   pl.ready = true;
   return KM_OK;
 }
@@ -229,18 +220,20 @@ inline int launch(Plan& pl, int* labels, IterState* st, bool count_changes, unsi
   const unsigned int seg_cap = (unsigned int)amb_seg_rows(pl.x_rows, num_sms);
   const bool pre = ensure_xsplit(pl, pl.x_base, pl.x_rows, pl.d, pl.sx, num_sms, stream, split_build);
   if (!pre) KM_TRY(ensure_xnorm(pl, pl.x_base, pl.x_rows, pl.d, num_sms, stream));
-  auto go = [&](auto fn, const CUtensorMap& tmX, bool p) {
+  auto go = [&](auto fn, const CUtensorMap& tmX, bool p) -> int {
+    KM_CUDA(allow_smem(fn, smem_bytes(pl.d, pl.npad, p)));
     fn<<<grid, kThreads, smem_bytes(pl.d, pl.npad, p), stream>>>(
         tmX, pl.tmBhi, pl.tmBlo, pl.cn, pl.xnorm, pl.xrowq, labels, pl.x_rows, (int)tiles, pl.npad, st,
         count_changes ? 1 : 0, amb_rows, amb_seg, seg_cap, tol_rel, tol_floor_of(pl.d), pl.sx, pl.sx * pl.sb,
         count_changes ? moved_bits : nullptr, amb_near, pre ? 1 : 0, wait_limits().mbar_iters);
     ++*launches;
+    return KM_OK;
   };
   if (pl.d == 32) {
-    go(assign_tc_kernel<32, false>, pl.tmX, false);
+    KM_TRY(go(assign_tc_kernel<32, false>, pl.tmX, false));
   } else {
-    if (pre) go(assign_tc_kernel<64, true>, pl.tmXh, true);
-    go(assign_tc_kernel<64, false>, pl.tmX, false);
+    if (pre) KM_TRY(go(assign_tc_kernel<64, true>, pl.tmXh, true));
+    KM_TRY(go(assign_tc_kernel<64, false>, pl.tmX, false));
   }
   KM_CUDA(cudaGetLastError());
   return KM_OK;
@@ -280,13 +273,6 @@ struct BigPlan {
 inline bool big_shape_ok(int k, int d) { return d >= 32 && d <= 256 && d % 4 == 0 && k > 16 && k <= 6144; }
 inline int big_variant(int d) { return d <= 32 ? 32 : (d <= 64 ? 64 : (d <= 128 ? 128 : 256)); }
 
-template <int D>
-inline int big_set_attr(int kpad) {
-  KM_CUDA(cudaFuncSetAttribute(assign_tc_big_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)big_smem_bytes<D>(kpad)));
-  return KM_OK;
-}
-
 // the operand table: upper and lower halves (float32) or upper halves only (float64)
 inline int big_tables(BigPlan& pl, int k, int d, bool lower) {
   const int kpad = (k + kNT - 1) / kNT * kNT;
@@ -308,13 +294,8 @@ inline int big_tables(BigPlan& pl, int k, int d, bool lower) {
 inline int big_setup(BigPlan& pl, const float* X, size_t rows, int k, int d, int ldx) {
   KM_TRY(big_tables(pl, k, d, true));
   if (pl.ready && pl.x_base == X && pl.x_rows == rows) return KM_OK;
-  const int kpad = pl.kpad, dv = big_variant(d);
   pl.x_base = X; pl.x_rows = rows;
   KM_TRY(tc::make_map(&pl.tmX, X, rows, ldx, kBM, 4));
-  if (dv == 32) KM_TRY(big_set_attr<32>(kpad));
-  else if (dv == 64) KM_TRY(big_set_attr<64>(kpad));
-  else if (dv == 128) KM_TRY(big_set_attr<128>(kpad));
-  else KM_TRY(big_set_attr<256>(kpad));
   pl.ready = true;
   return KM_OK;
 }
@@ -329,11 +310,14 @@ inline int big_prep(BigPlan& pl, const T* C, const T* cnorm, cudaStream_t stream
 }
 
 template <int D>
-inline void big_launch_d(BigPlan& pl, const float* xnorm, int xnorm_pitch, int* labels, IterState* st, int count_changes,
-                         unsigned int* amb_rows, float tol_rel, int grid, int tiles, cudaStream_t stream, int gate) {
+inline int big_launch_d(BigPlan& pl, const float* xnorm, int xnorm_pitch, int* labels, IterState* st, int count_changes,
+                        unsigned int* amb_rows, float tol_rel, int grid, int tiles, cudaStream_t stream, int gate) {
+  KM_CUDA(allow_smem(assign_tc_big_kernel<D>, big_smem_bytes<D>(pl.kpad)));
   assign_tc_big_kernel<D><<<grid, kBigThreads, big_smem_bytes<D>(pl.kpad), stream>>>(
       pl.tmX, pl.tmBhi, pl.tmBlo, pl.cn, xnorm, xnorm_pitch, labels, pl.x_rows, tiles, pl.kpad, st, count_changes,
       amb_rows, tol_rel, tc::tol_floor_of(pl.d), pl.sx, pl.sx * pl.sb, gate, wait_limits().mbar_iters);
+  KM_CUDA(cudaGetLastError());
+  return KM_OK;
 }
 
 // gate: the kernel returns at once unless the one-product kernel in front of it gave the pass up; xnorm_pitch: floats
@@ -345,12 +329,11 @@ inline int big_launch(BigPlan& pl, const float* xnorm, int xnorm_pitch, int* lab
   const int grid = (int)std::min<size_t>(tiles, (size_t)num_sms);
   const int cc = count_changes ? 1 : 0;
   const int dv = big_variant(pl.d);
-  if (dv == 32) big_launch_d<32>(pl, xnorm, xnorm_pitch, labels, st, cc, amb_rows, tol_rel, grid, (int)tiles, stream, gate ? 1 : 0);
-  else if (dv == 64) big_launch_d<64>(pl, xnorm, xnorm_pitch, labels, st, cc, amb_rows, tol_rel, grid, (int)tiles, stream, gate ? 1 : 0);
-  else if (dv == 128) big_launch_d<128>(pl, xnorm, xnorm_pitch, labels, st, cc, amb_rows, tol_rel, grid, (int)tiles, stream, gate ? 1 : 0);
-  else big_launch_d<256>(pl, xnorm, xnorm_pitch, labels, st, cc, amb_rows, tol_rel, grid, (int)tiles, stream, gate ? 1 : 0);
-  KM_CUDA(cudaGetLastError());
-  return KM_OK;
+  auto go = [&](auto fn) {
+    return fn(pl, xnorm, xnorm_pitch, labels, st, cc, amb_rows, tol_rel, grid, (int)tiles, stream, gate ? 1 : 0);
+  };
+  return dv == 32 ? go(big_launch_d<32>) : dv == 64 ? go(big_launch_d<64>)
+       : dv == 128 ? go(big_launch_d<128>) : go(big_launch_d<256>);
 }
 
 }  // namespace tcb
@@ -440,7 +423,7 @@ inline int half_launch_p(HalfPlan& pl, tcb::BigPlan& tb, int* labels, IterState*
   const size_t n_sub = (pl.rows + kBM - 1) / kBM;
   const int grid = (int)std::min<size_t>(n_sub, (size_t)num_sms);
   const size_t smem = half_smem_bytes(tb.d, tb.kpad);
-  KM_CUDA(cudaFuncSetAttribute(assign_tc_half_kernel<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  KM_CUDA(allow_smem(assign_tc_half_kernel<P>, smem));
   // rows whose candidates cannot be told apart by chunk cost k / 32 times more in the exact pass; what takes over
   // costs three times the one-product pass for float32 rows and forty times as much for float64 ones
   const unsigned int all_limit = (unsigned int)std::max<size_t>(64, tb.blo ? pl.rows / 64 : pl.rows / 8);
@@ -518,8 +501,6 @@ inline int wide_setup(WidePlan& pl, const float* X, size_t rows, int k, int d, i
   KM_TRY(tc::make_map(&pl.tmX, X, rows, ldx, kBM, 4));
   KM_TRY(tc::make_map(&pl.tmBhi, pl.bhi, kNPad, dp, kNPad, 2));
   KM_TRY(tc::make_map(&pl.tmBlo, pl.blo, kNPad, dp, kNPad, 2));
-  KM_CUDA(cudaFuncSetAttribute(assign_tc_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)wide_smem_bytes(n_chunks, pl.stages)));
   pl.ready = true;
   return KM_OK;
 }
@@ -541,6 +522,7 @@ inline int wide_launch(WidePlan& pl, const float* xnorm, int* labels, IterState*
   const size_t tiles = (nrows + kBM - 1) / kBM;
   if ((pl.x_rows + kBM - 1) / kBM > 0x7fffffffULL / kBM) KM_FAIL(KM_EINVAL, "shard too large for the tensor-core kernel");
   const int grid = (int)std::min<size_t>(tiles, (size_t)num_sms);
+  KM_CUDA(allow_smem(assign_tc_wide_kernel, wide_smem_bytes(pl.n_chunks, pl.stages)));
   assign_tc_wide_kernel<<<grid, kWThreads, wide_smem_bytes(pl.n_chunks, pl.stages), stream>>>(
       pl.tmX, pl.tmBhi, pl.tmBlo, pl.cn, xnorm, labels, std::min(pl.x_rows, row0 + nrows), (int)(row0 / kBM), (int)tiles,
       pl.n_chunks, pl.stages, pl.k, st, count_changes ? 1 : 0, amb_rows, tol_rel, tc::tol_floor_of(pl.d), pl.sx,
@@ -598,12 +580,6 @@ inline int stream_setup(StreamPlan& pl, const float* X, size_t rows, int k, int 
   KM_TRY(tc::make_map(&pl.tmX, X, rows, ldx, kBM, 4));
   KM_TRY(tc::make_map(&pl.tmBhi, pl.bhi, kpad, dp, npad, 2));
   KM_TRY(tc::make_map(&pl.tmBlo, pl.blo, kpad, dp, npad, 2));
-  if (npad == 128)
-    KM_CUDA(cudaFuncSetAttribute(assign_tc_stream_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)stream_smem_bytes<128>()));
-  else
-    KM_CUDA(cudaFuncSetAttribute(assign_tc_stream_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)stream_smem_bytes<256>()));
   pl.ready = true;
   return KM_OK;
 }
@@ -626,16 +602,19 @@ inline int stream_launch(StreamPlan& pl, const float* xnorm, int* labels, IterSt
   if ((pl.x_rows + kBM - 1) / kBM > 0x7fffffffULL / kBM) KM_FAIL(KM_EINVAL, "shard too large for the tensor-core kernel");
   const int grid = (int)std::min<size_t>(tiles, (size_t)num_sms);
   const size_t n_end = std::min(pl.x_rows, row0 + nrows);
-  if (pl.npad == 128)
+  if (pl.npad == 128) {
+    KM_CUDA(allow_smem(assign_tc_stream_kernel<128>, stream_smem_bytes<128>()));
     assign_tc_stream_kernel<128><<<grid, kSThreads, stream_smem_bytes<128>(), stream>>>(
         pl.tmX, pl.tmBhi, pl.tmBlo, pl.cn, xnorm, labels, n_end, (int)(row0 / kBM), (int)tiles, pl.n_chunks, pl.n_pass,
         pl.k, st, count_changes ? 1 : 0, amb_rows, tol_rel, tc::tol_floor_of(pl.d), pl.sx, pl.sx * pl.sb,
         wait_limits().mbar_iters, out, ld_out);
-  else
+  } else {
+    KM_CUDA(allow_smem(assign_tc_stream_kernel<256>, stream_smem_bytes<256>()));
     assign_tc_stream_kernel<256><<<grid, kSThreads, stream_smem_bytes<256>(), stream>>>(
         pl.tmX, pl.tmBhi, pl.tmBlo, pl.cn, xnorm, labels, n_end, (int)(row0 / kBM), (int)tiles, pl.n_chunks, pl.n_pass,
         pl.k, st, count_changes ? 1 : 0, amb_rows, tol_rel, tc::tol_floor_of(pl.d), pl.sx, pl.sx * pl.sb,
         wait_limits().mbar_iters, out, ld_out);
+  }
   KM_CUDA(cudaGetLastError());
   return KM_OK;
 }

@@ -1593,3 +1593,29 @@ def test_a_fit_that_fits_without_the_rounded_rows_runs(eng, built_lib, dtype, d,
         assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1]), extra
     with pytest.raises(lib_kmeans.KMeansLibError):
         fit(n * 8)
+
+
+# ---- several live handles ----------------------------------------------------------------------------
+@pytest.mark.parametrize("dtype,n,d,ks", [(np.float32, 3000, 64, (100, 20)), (np.float32, 3000, 32, (128, 17)),
+                                          (np.float32, 3000, 256, (2000, 20)), (np.float32, 20_000, 256, (3000, 400)),
+                                          (np.float64, 20_000, 128, (3000, 40)), (np.float64, 3000, 5, (900, 20)),
+                                          (np.float32, 3000, 784, (16, 3)), (np.float32, 3000, 7, (16, 2)),
+                                          (np.float64, 3000, 12, (16, 2))])
+def test_handles_with_many_and_few_centroids_alternate(eng, dtype, n, d, ks):
+    """Shared-memory limits belong to a kernel, not to a handle: a fit with few centroids on one handle must not take
+    away what the next fit with many on another one needs.  Same results as alone, fit after fit."""
+    rng = np.random.default_rng(d)
+    X = rng.uniform(-5, 5, (n, d)).astype(dtype)
+    hs, want = [], []
+    for k in ks:
+        h = eng.ResidentKMeans(dtype=dtype)
+        h.upload(X)
+        h.fit(X[:k].copy(), 2)
+        hs.append(h)
+        want.append((h.centroids(), h.labels()))
+    for _ in range(2):
+        for h, k, w in zip(hs, ks, want):
+            h.fit(X[:k].copy(), 2)
+            assert np.array_equal(h.centroids(), w[0]) and np.array_equal(h.labels(), w[1])
+    for h in hs:
+        h.close()
