@@ -352,17 +352,18 @@ rownorm_kernel(const float* __restrict__ X, size_t n, int d, float* __restrict__
 // padding rows; cn_pad[npad] = max_j |c_j|^2 (unscaled; zeroed before the launch).
 __global__ void __launch_bounds__(64)
 prep_kernel(const float* __restrict__ C, const float* __restrict__ cnorm, int k, int d, int npad, float sb,
-            float sxsb, __half* __restrict__ bhi, __half* __restrict__ blo, float* __restrict__ cn_pad) {
+            float sxsb, __half* __restrict__ bhi, __half* __restrict__ blo, float* __restrict__ cn_pad, OutRule rule) {
   const int j = blockIdx.x;
   const int t = threadIdx.x;  // 64 threads = 64 columns
-  float v = (j < k && t < d) ? -2.0f * C[(size_t)j * d + t] * sb : 0.0f;
+  const bool out = j >= k || left_out(rule, C + (size_t)j * d, d, cnorm, j, k);
+  float v = (!out && t < d) ? -2.0f * C[(size_t)j * d + t] * sb : 0.0f;
   const __half h = __float2half_rn(v);
   bhi[(size_t)j * 64 + t] = h;
   blo[(size_t)j * 64 + t] = __float2half_rn(v - __half2float(h));
   if (t == 0) {
-    cn_pad[j] = (j < k) ? cnorm[j] * sxsb : __int_as_float(0x7f800000);
+    cn_pad[j] = out ? __int_as_float(0x7f800000) : cnorm[j] * sxsb;
     // non-negative floats order as ints
-    if (j < k) atomicMax(reinterpret_cast<int*>(cn_pad + npad), __float_as_int(cnorm[j]));
+    if (!out) atomicMax(reinterpret_cast<int*>(cn_pad + npad), __float_as_int(cnorm[j]));
   }
 }
 

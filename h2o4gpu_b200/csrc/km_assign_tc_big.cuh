@@ -59,11 +59,12 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 big_prep_kernel(const T* __restrict__ C, const T* __restrict__ cnorm, int k, int d, int dp, int kpad,
                 float sb, float sxsb, __half* __restrict__ bhi, __half* __restrict__ blo,
-                float* __restrict__ cn_pad, const float* eb) {
+                float* __restrict__ cn_pad, const float* eb, OutRule rule) {
   const int j = blockIdx.x;
+  const bool out = j >= k || left_out(rule, C + (size_t)j * d, d, cnorm, j, k);
   double left = 0;
   for (int t = threadIdx.x; t < dp; t += blockDim.x) {
-    const T v = (j < k && t < d) ? (T)-2 * C[(size_t)j * d + t] * (T)sb : (T)0;
+    const T v = (!out && t < d) ? (T)-2 * C[(size_t)j * d + t] * (T)sb : (T)0;
     const __half h = to_half(v);
     const T r = v - (T)__half2float(h);   // exact
     bhi[(size_t)j * dp + t] = h;
@@ -71,8 +72,8 @@ big_prep_kernel(const T* __restrict__ C, const T* __restrict__ cnorm, int k, int
     left = fma((double)r, (double)r, left);
   }
   if (threadIdx.x == 0) {
-    cn_pad[j] = (j < k) ? (float)cnorm[j] * sxsb : __int_as_float(0x7f800000);
-    if (j < k) atomicMax(reinterpret_cast<int*>(cn_pad + kpad), __float_as_int((float)cnorm[j]));
+    cn_pad[j] = out ? __int_as_float(0x7f800000) : (float)cnorm[j] * sxsb;
+    if (!out) atomicMax(reinterpret_cast<int*>(cn_pad + kpad), __float_as_int((float)cnorm[j]));
   }
   if (eb) {
     __shared__ double part[8];

@@ -5,6 +5,7 @@
 #include <cuda_fp16.h>
 #include <algorithm>
 #include <cstdlib>
+#include <limits>
 #include <map>
 #include <mutex>
 #include <utility>
@@ -338,6 +339,37 @@ __device__ __forceinline__ double warp_sum(double v) {
 // one rounding to fp16, to nearest
 __device__ __forceinline__ __half to_half(float v) { return __float2half_rn(v); }
 __device__ __forceinline__ __half to_half(double v) { return __double2half(v); }
+
+// Centroids that no row can be nearest to, and that the operand tables of the tensor-core kernels therefore leave out
+// (as padding rows).  With |x_t| <= xmax and R^2 = d xmax^2 >= |x|^2, and another centroid c' with |c'| <= R:
+//   |x - c|^2 - |x - c'|^2 = |c|^2 - |c'|^2 - 2 x.c + 2 x.c' >= |c|^2 - 2 xmax |c|_1 - 3 R^2,
+// so c is out once that is positive.  A cluster that stays empty takes the unscaled sums of the largest one and can
+// lie that far outside the data, where its fp16 operands would overflow and the error bounds of all rows, which
+// grow with the longest centroid, would open every row.
+struct OutRule {
+  float two_xmax = 0.f;                     // 2 xmax and 3 R^2, a little more of each
+  float three_rr = std::numeric_limits<float>::infinity();   // (off by default)
+  float rr = 0.f;
+  __device__ __forceinline__ bool operator()(float cn, float l1) const { return cn > fmaf(two_xmax, l1, three_rr); }
+};
+inline OutRule out_rule(double xmax, int d) {
+  OutRule r;
+  const double rr = (double)d * xmax * xmax;
+  if (rr < 1e37) { r.two_xmax = (float)(2.01 * xmax); r.three_rr = (float)(3.05 * rr); r.rr = (float)rr; }
+  return r;
+}
+// Whether the CTA's centroid `c` (row j of a table of k) is left out.  Called by every thread of the CTA.  A table that
+// comes from the caller need not hold a centroid within R (the mean of any cluster with members lies there).
+template <typename T>
+__device__ bool left_out(const OutRule& rule, const T* __restrict__ c, int d, const T* __restrict__ cnorm, int j, int k) {
+  if (!rule((float)cnorm[j], 0.f)) return false;   // all but a few: no need for |c|_1
+  float l1 = 0.f;
+  for (int t = 0; t < d; ++t) l1 += fabsf((float)c[t]);
+  if (!rule((float)cnorm[j], l1)) return false;
+  for (int i = 0; i < k; ++i)
+    if ((float)cnorm[i] <= rule.rr) return true;
+  return false;
+}
 
 template <typename T> struct Inf;
 template <> struct Inf<float> { __device__ static float v() { return __int_as_float(0x7f800000); } };

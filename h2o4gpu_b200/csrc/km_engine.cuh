@@ -101,6 +101,7 @@ struct Shard {
   tcb::BigPlan tcbp;  // tensor-core path for large centroid tables
   tch::HalfPlan tchp; // one-product kernel on rounded rows (large tables; float64)
   tcw::WidePlan tcwp; // tensor-core path for few centroids and wide rows
+  int estep_kernel = 0;   // label kernel of the last pass (kmeans_estep_info)
   tcs::StreamPlan tcsp;  // tensor-core path with both operands streamed: wide rows and many centroids, transform
   unsigned int* amb_rows = nullptr;  // rows handed to the exact re-evaluation pass
   T* xpad = nullptr;                 // rows padded to a multiple of four columns (d % 4 != 0): what TMA can address
@@ -285,8 +286,10 @@ struct Engine : EngineBase {
     return KM_OK;
   }
   const T* xtc(const Shard<T>& s) const { return d % 4 == 0 ? s.X : s.xpad; }
-  int stream_refresh(Shard<T>& s);   // operand table and plan of the streaming kernel for the current centroids
-  int tc_refresh(Shard<T>& s);  // split the current centroids for the tensor-core kernel
+  int stream_refresh(Shard<T>& s, const OutRule& rule);   // operand table and plan of the streaming kernel for the current centroids
+  // split the current centroids for the tensor-core kernel; for labels the table leaves out those that no row can be
+  // nearest to
+  int tc_refresh(Shard<T>& s, bool for_labels = true);
   int launch_assign(Shard<T>& s, bool use_tc, bool count_changes);
   tc::SplitBuild tc_split_build = tc::SplitBuild::no;   // whether the running fit pays for the split copy of X
   // Begins a call that labels rows.  The caller may have written other values into a matrix it lends
@@ -299,6 +302,11 @@ struct Engine : EngineBase {
       s.tchp.of = nullptr;
       if (!s.tcp.xsplit_kept) s.tcp.xsplit_of = nullptr;
     }
+  }
+  double xmax_all() const {
+    double m = 0;
+    for (const auto& s : shards) m = std::max(m, s.xmax);
+    return m;
   }
   float tc_sx = 1.f, tc_sb = 1.f;   // operand scales of the tensor-core kernel
   double cbound = 0;                // bound on |centroid coordinate|: max(|x|, |initial centroids|)
@@ -1354,7 +1362,8 @@ bool Engine<T>::tc_ok(int flags) const {
 }
 
 template <typename T>
-int Engine<T>::tc_refresh(Shard<T>& s) {
+int Engine<T>::tc_refresh(Shard<T>& s, bool for_labels) {
+  const OutRule rule = for_labels ? out_rule(xmax_all(), d) : OutRule{};
   const bool half = half_shape_ok() && (tc_kind() == 2 || tc_kind() == 5);
   s.tchp.on = false;
   if constexpr (std::is_same<T, double>::value) {
@@ -1366,7 +1375,7 @@ int Engine<T>::tc_refresh(Shard<T>& s) {
     KM_TRY(tcb::big_tables(s.tcbp, k, d, false));
     s.tcbp.sx = tc_sx;
     s.tcbp.sb = tc_sb;
-    KM_TRY(tcb::big_prep(s.tcbp, s.C[cur], s.cnorm, s.stream));
+    KM_TRY(tcb::big_prep(s.tcbp, s.C[cur], s.cnorm, rule, s.stream));
     ++launches;
   } else {
     double xmax = 0;
@@ -1388,21 +1397,21 @@ int Engine<T>::tc_refresh(Shard<T>& s) {
       KM_TRY(tcw::wide_setup(s.tcwp, xtc(s), s.rows, k, d, dtc()));
       s.tcwp.sx = tc_sx;
       s.tcwp.sb = tc_sb;
-      KM_TRY(tcw::wide_prep(s.tcwp, s.C[cur], s.cnorm, s.stream));
+      KM_TRY(tcw::wide_prep(s.tcwp, s.C[cur], s.cnorm, rule, s.stream));
     } else if (kind == 4) {
-      KM_TRY(stream_refresh(s));
+      KM_TRY(stream_refresh(s, rule));
     } else if (kind == 1) {
       KM_TRY(tc::setup(s.tcp, s.X, s.rows, k, d, s.num_sms, s.stream));
       s.tcp.sx = tc_sx;
       s.tcp.sb = tc_sb;
-      KM_TRY(tc::prep(s.tcp, s.C[cur], s.cnorm, s.stream));
+      KM_TRY(tc::prep(s.tcp, s.C[cur], s.cnorm, rule, s.stream));
     } else {
       if (!s.tchp.on)
         KM_TRY(tc::ensure_xnorm(s.tcp, xtc(s), s.rows, dtc(), s.num_sms, s.stream));   // float4 loads: the aligned rows
       KM_TRY(tcb::big_setup(s.tcbp, xtc(s), s.rows, k, d, dtc()));
       s.tcbp.sx = tc_sx;
       s.tcbp.sb = tc_sb;
-      KM_TRY(tcb::big_prep(s.tcbp, s.C[cur], s.cnorm, s.stream));
+      KM_TRY(tcb::big_prep(s.tcbp, s.C[cur], s.cnorm, rule, s.stream));
     }
     ++launches;
   }
@@ -1443,20 +1452,21 @@ int Engine<T>::ensure_xpad(Shard<T>& s, bool fill) {
 }
 
 template <typename T>
-int Engine<T>::stream_refresh(Shard<T>& s) {
+int Engine<T>::stream_refresh(Shard<T>& s, const OutRule& rule) {
   if constexpr (std::is_same<T, float>::value) {
     if (d % 4 != 0) KM_TRY(ensure_xpad(s));
     KM_TRY(tc::ensure_xnorm(s.tcp, xtc(s), s.rows, dtc(), s.num_sms, s.stream));   // float4 loads: the aligned rows
     KM_TRY(tcs::stream_setup(s.tcsp, xtc(s), s.rows, k, d, dtc()));
     s.tcsp.sx = tc_sx;
     s.tcsp.sb = tc_sb;
-    KM_TRY(tcs::stream_prep(s.tcsp, s.C[cur], s.cnorm, s.stream));
+    KM_TRY(tcs::stream_prep(s.tcsp, s.C[cur], s.cnorm, rule, s.stream));
   }
   return KM_OK;
 }
 
 template <typename T>
 int Engine<T>::launch_assign(Shard<T>& s, bool use_tc, bool count_changes) {
+  s.estep_kernel = !use_tc ? 0 : tc_kind() == 2 && s.tchp.on ? 5 : tc_kind() == 5 && !s.tchp.on ? 0 : tc_kind();
   if constexpr (std::is_same<T, float>::value) {
     if (use_tc && tc_kind() == 4) {
       launches += 2;

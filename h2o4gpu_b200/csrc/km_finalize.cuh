@@ -631,27 +631,22 @@ struct SplitTable {
   float* eb;
   int npad, dp;
   float sb, sxsb;
-  // |c|^2 above which a centroid cannot be the nearest of any row: with R = sqrt(d) max|x| >= |x| and another
-  // centroid inside R (the mean of any cluster with members), |x - c| > 2 R once |c| > 3 R.  Such a centroid exists:
-  // a cluster that stays empty takes the unscaled sums of the largest one.  It enters the table as a padding row -
-  // its fp16 halves would overflow, and the error bounds of all rows grow with the longest centroid.
-  float far_sq;
+  OutRule out;   // centroids it leaves out
 };
 
 // returns this thread's share of the squared length of what the upper halves leave out
 template <typename T>
-__device__ __forceinline__ double split_table_row(const SplitTable& tp, int j, int d, const T* c_row, T cn) {
+__device__ __forceinline__ double split_table_row(const SplitTable& tp, int j, int d, const T* c_row, T cn, bool out) {
   double left = 0;
-  const bool far = (float)cn > tp.far_sq;
   for (int t = threadIdx.x; t < tp.dp; t += blockDim.x) {
-    const T v = (t < d && !far) ? (T)-2 * c_row[t] * (T)tp.sb : (T)0;
+    const T v = (t < d && !out) ? (T)-2 * c_row[t] * (T)tp.sb : (T)0;
     const __half h = to_half(v);
     const T r = v - (T)__half2float(h);   // exact
     tp.bhi[(size_t)j * tp.dp + t] = h;
     if (tp.blo) tp.blo[(size_t)j * tp.dp + t] = to_half(r);
     left = fma((double)r, (double)r, left);
   }
-  if (threadIdx.x == 0) tp.cn_pad[j] = far ? __int_as_float(0x7f800000) : (float)cn * tp.sxsb;
+  if (threadIdx.x == 0) tp.cn_pad[j] = out ? __int_as_float(0x7f800000) : (float)cn * tp.sxsb;
   return left;
 }
 
@@ -681,6 +676,7 @@ close_kernel(const long long* __restrict__ gsums, const unsigned long long* __re
   const int n_empty = st->n_empty;
   if ((run_if == 0 && n_empty != 0) || (run_if == 1 && n_empty == 0)) return;
   __shared__ double red_n[4], red_s[4];
+  __shared__ float red_l[4];
   __shared__ int s_src, s_last;
   const int j = blockIdx.x;
   unsigned long long cnt = gcounts[j];
@@ -706,6 +702,7 @@ close_kernel(const long long* __restrict__ gsums, const unsigned long long* __re
     a = (src < j && cb > 0) ? 1.0 / ((double)cb * count_unit) : 1.0;
   }
   double sn = 0, ss = 0;
+  float sl = 0;
   for (int t = threadIdx.x; t < d; t += blockDim.x) {
     long long g[NP / 2];
 #pragma unroll
@@ -717,10 +714,14 @@ close_kernel(const long long* __restrict__ gsums, const unsigned long long* __re
     double df = dv - (double)C_old[(size_t)j * d + t];
     sn += dv * dv;
     ss += df * df;
+    sl += fabsf((float)v);
   }
   sn = warp_sum(sn);
   ss = warp_sum(ss);
-  if ((threadIdx.x & 31) == 0) { red_n[threadIdx.x >> 5] = sn; red_s[threadIdx.x >> 5] = ss; }
+  // only a cluster without members can lie outside the data
+  if (cnt == 0)
+    for (int o = 16; o > 0; o >>= 1) sl += __shfl_xor_sync(0xffffffffu, sl, o);
+  if ((threadIdx.x & 31) == 0) { red_n[threadIdx.x >> 5] = sn; red_s[threadIdx.x >> 5] = ss; red_l[threadIdx.x >> 5] = sl; }
   __syncthreads();
   const T cn = (T)(red_n[0] + red_n[1] + red_n[2] + red_n[3]);
   if (threadIdx.x == 0) {
@@ -729,7 +730,8 @@ close_kernel(const long long* __restrict__ gsums, const unsigned long long* __re
   }
   if (tp.bhi != nullptr) {
     __syncthreads();   // the row of C_new written above is read back by other threads
-    const double left = split_table_row<T>(tp, j, d, C_new + (size_t)j * d, cn);
+    const bool out = cnt == 0 && tp.out((float)cn, red_l[0] + red_l[1] + red_l[2] + red_l[3]);
+    const double left = split_table_row<T>(tp, j, d, C_new + (size_t)j * d, cn, out);
     if (tp.eb != nullptr) {
       const double w = warp_sum(left);
       if ((threadIdx.x & 31) == 0) red_n[threadIdx.x >> 5] = w;
@@ -750,10 +752,7 @@ close_kernel(const long long* __restrict__ gsums, const unsigned long long* __re
   float m = 0.f, meb = 0.f;
   for (int c = threadIdx.x; c < k; c += 128) {
     s += __ldcg(shift_k + c);
-    if (tp.bhi != nullptr) {
-      const float cn_c = (float)__ldcg(cnorm + c);
-      if (!(cn_c > tp.far_sq)) m = fmaxf(m, cn_c);
-    }
+    if (tp.bhi != nullptr && __ldcg(tp.cn_pad + c) < __int_as_float(0x7f800000)) m = fmaxf(m, (float)__ldcg(cnorm + c));
     if (tp.eb != nullptr) meb = fmaxf(meb, __ldcg(tp.eb + c));
   }
   __shared__ float rede[128];

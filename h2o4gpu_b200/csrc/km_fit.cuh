@@ -130,21 +130,19 @@ int Engine<T>::relocate_multi(double scale, int seq, int* n_empty) {
 
 template <typename T>
 SplitTable Engine<T>::split_table(Shard<T>& s, bool use_tc) {
-  double xmax = 0;
-  for (const auto& sh : shards) xmax = std::max(xmax, sh.xmax);
-  const float far_sq = (float)(9.1 * d * xmax * xmax);
-  SplitTable tp{nullptr, nullptr, nullptr, nullptr, 0, 0, 0.f, 0.f, far_sq};
+  const OutRule out = out_rule(xmax_all(), d);
+  SplitTable tp{nullptr, nullptr, nullptr, nullptr, 0, 0, 0.f, 0.f, out};
   if constexpr (std::is_same<T, float>::value) {
     if (use_tc && tc_kind() == 4)
-      tp = SplitTable{s.tcsp.bhi, s.tcsp.blo, s.tcsp.cn, nullptr, s.tcsp.kpad, s.tcsp.dp, s.tcsp.sb, s.tcsp.sx * s.tcsp.sb, far_sq};
+      tp = SplitTable{s.tcsp.bhi, s.tcsp.blo, s.tcsp.cn, nullptr, s.tcsp.kpad, s.tcsp.dp, s.tcsp.sb, s.tcsp.sx * s.tcsp.sb, out};
     else if (use_tc && tc_kind() == 3)
-      tp = SplitTable{s.tcwp.bhi, s.tcwp.blo, s.tcwp.cn, nullptr, tcw::kNPad, s.tcwp.dp, s.tcwp.sb, s.tcwp.sx * s.tcwp.sb, far_sq};
+      tp = SplitTable{s.tcwp.bhi, s.tcwp.blo, s.tcwp.cn, nullptr, tcw::kNPad, s.tcwp.dp, s.tcwp.sb, s.tcwp.sx * s.tcwp.sb, out};
     else if (use_tc && tc_kind() == 1)
-      tp = SplitTable{s.tcp.bhi, s.tcp.blo, s.tcp.cn, nullptr, s.tcp.npad, 64, s.tcp.sb, s.tcp.sx * s.tcp.sb, far_sq};
+      tp = SplitTable{s.tcp.bhi, s.tcp.blo, s.tcp.cn, nullptr, s.tcp.npad, 64, s.tcp.sb, s.tcp.sx * s.tcp.sb, out};
   }
   if (!tp.bhi && use_tc && (tc_kind() == 2 || s.tchp.on))
     tp = SplitTable{s.tcbp.bhi, s.tcbp.blo, s.tcbp.cn, s.tcbp.eb, s.tcbp.kpad, s.tcbp.dp, s.tcbp.sb,
-                    s.tcbp.sx * s.tcbp.sb, far_sq};
+                    s.tcbp.sx * s.tcbp.sb, out};
   return tp;
 }
 
@@ -561,17 +559,17 @@ int Engine<T>::transform_shard(int local, T* out_host, size_t ld) {
     // tensor-core kernels with a store epilogue (they need max|x| for the operand scales, i.e. a checked
     // matrix): the wide-row kernel for few centroids, the kernel that streams both operands for the rest
     if (tc_kind() == 3 && tc_ok(0)) {
-      rc = tc_refresh(s);
+      rc = tc_refresh(s, false);
       wide = rc == KM_OK;
     } else if (tcs::stream_shape_ok(k, dtc()) && tc_ok(0)) {
       if (tc_kind() == 4) {
-        rc = tc_refresh(s);
+        rc = tc_refresh(s, false);
       } else {
         // the shape's own labelling kernel keeps its plan; the streaming kernel gets one beside it
         double xmax = 0;
         for (const auto& sh : shards) xmax = std::max(xmax, sh.xmax);
         if (!tc::pick_scales(xmax, std::max(xmax, cbound), &tc_sx, &tc_sb)) rc = KM_EINVAL;
-        if (rc == KM_OK) rc = stream_refresh(s);
+        if (rc == KM_OK) rc = stream_refresh(s, OutRule{});
         if (rc == KM_OK) ++launches;
       }
       streamed = rc == KM_OK;

@@ -179,9 +179,11 @@ inline int setup(Plan& pl, const float* X, size_t rows, int k, int d, int num_sm
   return KM_OK;
 }
 
-inline int prep(Plan& pl, const float* C, const float* cnorm, cudaStream_t stream) {
+// rule: centroids the table leaves out (none for distances, which are wanted for all)
+inline int prep(Plan& pl, const float* C, const float* cnorm, const OutRule& rule, cudaStream_t stream) {
   KM_CUDA(cudaMemsetAsync(pl.cn + pl.npad, 0, sizeof(float), stream));
-  prep_kernel<<<pl.npad, 64, 0, stream>>>(C, cnorm, pl.k, pl.d, pl.npad, pl.sb, pl.sx * pl.sb, pl.bhi, pl.blo, pl.cn);
+  prep_kernel<<<pl.npad, 64, 0, stream>>>(C, cnorm, pl.k, pl.d, pl.npad, pl.sb, pl.sx * pl.sb, pl.bhi, pl.blo, pl.cn,
+                                         rule);
   KM_CUDA(cudaGetLastError());
   return KM_OK;
 }
@@ -301,10 +303,10 @@ inline int big_setup(BigPlan& pl, const float* X, size_t rows, int k, int d, int
 }
 
 template <typename T>
-inline int big_prep(BigPlan& pl, const T* C, const T* cnorm, cudaStream_t stream) {
+inline int big_prep(BigPlan& pl, const T* C, const T* cnorm, const OutRule& rule, cudaStream_t stream) {
   KM_CUDA(cudaMemsetAsync(pl.cn + pl.kpad, 0, 2 * sizeof(float), stream));
   big_prep_kernel<T><<<pl.kpad, 256, 0, stream>>>(C, cnorm, pl.k, pl.d, pl.dp, pl.kpad, pl.sb, pl.sx * pl.sb, pl.bhi,
-                                                  pl.blo, pl.cn, pl.eb);
+                                                  pl.blo, pl.cn, pl.eb, rule);
   KM_CUDA(cudaGetLastError());
   return KM_OK;
 }
@@ -505,10 +507,10 @@ inline int wide_setup(WidePlan& pl, const float* X, size_t rows, int k, int d, i
   return KM_OK;
 }
 
-inline int wide_prep(WidePlan& pl, const float* C, const float* cnorm, cudaStream_t stream) {
+inline int wide_prep(WidePlan& pl, const float* C, const float* cnorm, const OutRule& rule, cudaStream_t stream) {
   KM_CUDA(cudaMemsetAsync(pl.cn + kNPad, 0, sizeof(float), stream));
   tcb::big_prep_kernel<float><<<kNPad, 256, 0, stream>>>(C, cnorm, pl.k, pl.d, pl.dp, kNPad, pl.sb, pl.sx * pl.sb,
-                                                         pl.bhi, pl.blo, pl.cn, nullptr);
+                                                         pl.bhi, pl.blo, pl.cn, nullptr, rule);
   KM_CUDA(cudaGetLastError());
   return KM_OK;
 }
@@ -584,10 +586,10 @@ inline int stream_setup(StreamPlan& pl, const float* X, size_t rows, int k, int 
   return KM_OK;
 }
 
-inline int stream_prep(StreamPlan& pl, const float* C, const float* cnorm, cudaStream_t stream) {
+inline int stream_prep(StreamPlan& pl, const float* C, const float* cnorm, const OutRule& rule, cudaStream_t stream) {
   KM_CUDA(cudaMemsetAsync(pl.cn + pl.kpad, 0, sizeof(float), stream));
   tcb::big_prep_kernel<float><<<pl.kpad, 256, 0, stream>>>(C, cnorm, pl.k, pl.d, pl.dp, pl.kpad, pl.sb, pl.sx * pl.sb,
-                                                          pl.bhi, pl.blo, pl.cn, nullptr);
+                                                          pl.bhi, pl.blo, pl.cn, nullptr, rule);
   KM_CUDA(cudaGetLastError());
   return KM_OK;
 }

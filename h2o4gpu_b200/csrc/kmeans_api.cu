@@ -386,6 +386,20 @@ static int get_stats(km::Engine<T>* e, kmeans_stats* out, int want_inertia) {
   return KM_OK;
 }
 
+// the label kernel of shard `local`'s last pass, and whether the device has sent that on to the one that reads whole rows
+template <typename T>
+static int estep_info(km::Engine<T>* e, int local, int* kernel, int* whole_rows) {
+  if (!kernel || !whole_rows || local < 0 || local >= (int)e->shards.size()) KM_FAIL(KM_EINVAL, "kmeans_estep_info: bad argument");
+  km::Shard<T>& s = e->shards[local];
+  km::DevGuard g(s.dev);
+  unsigned int w = 0;
+  KM_CUDA(cudaMemcpyAsync(&w, &s.st->full_rows, sizeof(w), cudaMemcpyDeviceToHost, s.stream));
+  KM_CUDA(cudaStreamSynchronize(s.stream));
+  *kernel = s.estep_kernel;
+  *whole_rows = w != 0;
+  return KM_OK;
+}
+
 // ---- extern "C" surface ---------------------------------------------------------
 extern "C" {
 
@@ -597,6 +611,9 @@ int kmeans_transform_resident(kmeans_handle_t h, int local, void* out, size_t ld
 
 int kmeans_get_stats(kmeans_handle_t h, kmeans_stats* out) {
   KM_DISPATCH(h, get_stats(h->f32, out, 0), get_stats(h->f64, out, 0));
+}
+int kmeans_estep_info(kmeans_handle_t h, int local, int* kernel, int* whole_rows) {
+  KM_DISPATCH(h, estep_info(h->f32, local, kernel, whole_rows), estep_info(h->f64, local, kernel, whole_rows));
 }
 int kmeans_inertia(kmeans_handle_t h, double* out) {
   if (!out) KM_FAIL(KM_EINVAL, "NULL output");

@@ -150,6 +150,13 @@ class ResidentKMeans(object):
         _lk.check(self._lib.kmeans_get_stats(self._h, ctypes.byref(st)))
         return st.as_dict()
 
+    def estep_info(self, local=0):
+        """(label kernel of the last pass, whether the device sent the pass on to whole rows); the numbers are those of
+        ``kmeans_estep_info`` in the header."""
+        kernel, whole = ctypes.c_int(), ctypes.c_int()
+        _lk.check(self._lib.kmeans_estep_info(self._h, local, ctypes.byref(kernel), ctypes.byref(whole)))
+        return kernel.value, bool(whole.value)
+
     def inertia(self):
         v = ctypes.c_double()
         _lk.check(self._lib.kmeans_inertia(self._h, ctypes.byref(v)))

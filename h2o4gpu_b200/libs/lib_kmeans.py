@@ -80,6 +80,7 @@ SIGNATURES = {
     "kmeans_labels_device": (_c.c_int, [_vp, _c.c_int, _c.POINTER(_vp)]),
     "kmeans_transform_resident": (_c.c_int, [_vp, _c.c_int, _vp, _sz]),
     "kmeans_get_stats": (_c.c_int, [_vp, _c.POINTER(Stats)]),
+    "kmeans_estep_info": (_c.c_int, [_vp, _c.c_int, _c.POINTER(_c.c_int), _c.POINTER(_c.c_int)]),
     "kmeans_inertia": (_c.c_int, [_vp, _c.POINTER(_c.c_double)]),
     "kmeans_centroid_sums_f32": (_c.c_int, [_c.c_int, _vp, _vp, _sz, _sz, _c.c_int, _vp, _vp]),
     "kmeans_centroid_sums_f64": (_c.c_int, [_c.c_int, _vp, _vp, _sz, _sz, _c.c_int, _vp, _vp]),

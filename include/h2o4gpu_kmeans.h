@@ -234,6 +234,12 @@ typedef struct kmeans_stats {
                             * over peer memory, 2 ncclAllReduce                                   */
 } kmeans_stats;
 int kmeans_get_stats(kmeans_handle_t h, kmeans_stats* out);
+/* Which kernel the last label pass over shard `local` ran (of a fit, or kmeans_assign_resident): 0 a SIMT
+ * kernel or the float64 matrix unit, 1 small table, 2 streamed table with three products per pair, 3 few centroids
+ * and wide rows, 4 both operands streamed, 5 one product per pair on rounded rows.  *whole_rows: 1 when rounded
+ * rows (kernels 1 and 5) left too many rows open and the device sent the pass on to the kernel that reads whole
+ * rows.  For tests and for a look at what a data set does. */
+int kmeans_estep_info(kmeans_handle_t h, int local, int* kernel, int* whole_rows);
 /* Sum of squared distances of every row to its assigned centre (direct
  * differences in double, all ranks): sklearn's inertia_, which the reference's
  * GPU path never sets (src/interface_py/h2o4gpu/solvers/kmeans.py:187). */

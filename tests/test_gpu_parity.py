@@ -1619,3 +1619,63 @@ def test_handles_with_many_and_few_centroids_alternate(eng, dtype, n, d, ks):
             assert np.array_equal(h.centroids(), w[0]) and np.array_equal(h.labels(), w[1])
     for h in hs:
         h.close()
+
+
+# ---- centroids far outside the data -----------------------------------------------------------------
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("dense", [False, True])
+def test_a_far_centroid_does_not_open_every_row(eng, dtype, dense):
+    """A cluster that stays empty takes the unscaled sums of the largest one.  Twenty equal sparse rows put it out of
+    the fp16 operands' range without putting it far away in length; dense rows put it far away.  No row can be nearest to
+    it, so it must not widen the bound of the others: neither the fit's E-steps nor its closing pass nor a later
+    assignment is sent on to whole rows, and the labels are the float64 argmin."""
+    rng = np.random.default_rng(11)
+    if dense:
+        pts, copies, last = rng.uniform(-5, 5, (400, 128)), 100, 300
+    else:
+        pts, copies, last = np.zeros((2000, 256)), 8, 20
+        for p in pts:
+            p[rng.choice(256, 4, replace=False)] = 1.0
+    X = np.concatenate([np.repeat(pts[:-1], copies, axis=0), np.repeat(pts[-1:], last, axis=0)]).astype(dtype)
+    # centroid 1 repeats centroid 0 and stays empty: every row lies on its own centroid, so there is none to take; the
+    # largest cluster comes later, so its sums are taken as they are
+    C = np.concatenate([pts[:1], pts]).astype(dtype)
+    h = eng.ResidentKMeans(dtype=dtype)
+    h.upload(X)
+    h.fit(C, 2)
+    got = h.centroids()
+    assert np.abs(got).max() > 4 * 2 * np.abs(X).max()
+    assert h.estep_info() == (5, False)
+    assert _nearest_gap(X, got, h.labels()) == 0
+    h.assign()
+    assert h.estep_info() == (5, False)
+    assert _nearest_gap(X, got, h.labels()) == 0
+    h.close()
+
+
+@pytest.mark.parametrize("dtype,n,d,k", [(np.float32, 20_000, 64, 100), (np.float32, 20_000, 128, 900),
+                                         (np.float32, 20_000, 784, 16), (np.float32, 20_000, 512, 600),
+                                         (np.float64, 20_000, 128, 900)])
+@pytest.mark.parametrize("all_far", [False, True])
+def test_far_centroids_of_the_caller_are_labelled_and_measured(eng, dtype, n, d, k, all_far):
+    """Tables with centroids up to 30 times as far out as the data, some of them or all: labels are the float64 argmin (a
+    table without a centroid near the data has its nearest among the far ones), and transform gives the distances to
+    the far ones too."""
+    rng = np.random.default_rng(d + k)
+    X = rng.uniform(-1, 1, (n, d)).astype(dtype)
+    C = rng.uniform(-1, 1, (k, d))
+    C[slice(None) if all_far else slice(0, None, 3)] *= 30
+    C = C.astype(dtype)
+    h = eng.ResidentKMeans(dtype=dtype)
+    h.upload(X)
+    h.set_centroids(C)
+    h.assign()
+    assert _nearest_gap(X, C, h.labels()) == 0
+    got = h.transform()
+    want = ((X[:500, None, :].astype(np.float64) - C[None].astype(np.float64)) ** 2).sum(2)
+    # scores of float32 rows: the split products' bound relative to |x|^2 + max |c|^2; float64: a few roundings of it
+    size = (X[:500].astype(np.float64) ** 2).sum(1).max() + (C.astype(np.float64) ** 2).sum(1).max()
+    assert np.abs(got[:500] - want).max() < (2.0 ** -18 * (0.8 + d / 200) if dtype == np.float32 else 1e-14) * size
+    h.assign()
+    assert _nearest_gap(X, C, h.labels()) == 0
+    h.close()
