@@ -387,8 +387,9 @@ struct IterState {
   unsigned int cand_all;        // ... of which all chunks may hold the nearest centroid
   unsigned int half_done;       // CTAs of the running one-product kernel that have finished (zero between launches)
   unsigned int full_rows;       // 1: an E-step on rounded rows left too many open for the exact pass; the fit goes on
-                                // with the kernel that reads the whole rows (cleared when a fit begins, data is attached)
-  unsigned int pad_ready;       // 1: the padded copy those need for unaligned rows has been filled (cleared alike)
+                                // with the kernel that reads the whole rows (cleared when centroids are set, data is attached)
+  unsigned int pad_ready;       // 1: the padded copy those need for unaligned rows has been filled (cleared when a fit
+                                // begins, data is attached)
   double shift_sq;              // summed squared centroid shift of the current M-step
   double inertia;               // scratch for the inertia pass
 };

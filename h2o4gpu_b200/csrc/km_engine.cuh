@@ -1108,6 +1108,8 @@ int Engine<T>::set_centroids(int k_, const T* host_c) {
   for (auto& s : shards) {
     DevGuard g(s.dev);
     KM_CUDA(cudaMemcpyAsync(s.C[0], host_c, (size_t)k * d * sizeof(T), cudaMemcpyHostToDevice, s.stream));
+    // another table may be less crowded than the one that sent the E-step on to whole rows
+    KM_CUDA(cudaMemsetAsync(&s.st->full_rows, 0, sizeof(unsigned int), s.stream));
     cnorm_kernel<T><<<k, 128, 0, s.stream>>>(s.C[0], k, d, s.cnorm, s.Cd[0]);
     KM_CUDA(cudaGetLastError());
     ++launches;

@@ -1679,3 +1679,25 @@ def test_far_centroids_of_the_caller_are_labelled_and_measured(eng, dtype, n, d,
     h.assign()
     assert _nearest_gap(X, C, h.labels()) == 0
     h.close()
+
+
+def test_a_crowded_table_does_not_slow_the_next_one(eng):
+    """What a table of centroids close together decides on the device (rounded rows leave every row open) ends with that
+    table: the next one on the same matrix runs on the rounded rows again."""
+    rng = np.random.default_rng(2)
+    for dtype, n, d, k in [(np.float32, 40_000, 64, 900), (np.float32, 40_000, 50, 600), (np.float64, 40_000, 64, 300)]:
+        centers = rng.uniform(-6, 6, (k, d))
+        X = (centers[rng.integers(0, k, n)] + rng.standard_normal((n, d))).astype(dtype)
+        crowded = (3.0 + 1e-5 * rng.standard_normal((k, d))).astype(dtype)
+        h = eng.ResidentKMeans(dtype=dtype)
+        h.upload(X)
+        for _ in range(2):
+            h.set_centroids(crowded)
+            h.assign()
+            assert h.estep_info() == (5, True)
+            assert _nearest_gap(X, crowded, h.labels()) == 0
+            h.set_centroids(centers)
+            h.assign()
+            assert h.estep_info() == (5, False)
+            assert _nearest_gap(X, centers.astype(dtype), h.labels()) == 0
+        h.close()
