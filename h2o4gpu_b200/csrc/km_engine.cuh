@@ -394,7 +394,6 @@ int Engine<T>::init(int n_local, const int* devs, int rank0, int world, const vo
     KM_CUDA(cudaMemset(s.ticket, 0, sizeof(unsigned int)));
     s.far.cap = 32768;
     KM_CUDA(km_malloc(&s.far.tmax, (size_t)s.num_sms * 256 * sizeof(double)));
-    KM_CUDA(km_malloc(&s.far.trow, (size_t)s.num_sms * 256 * sizeof(unsigned long long)));
     KM_CUDA(km_malloc(&s.far.cval, (size_t)s.far.cap * sizeof(double)));
     KM_CUDA(km_malloc(&s.far.crow, (size_t)s.far.cap * sizeof(unsigned long long)));
     KM_CUDA(km_malloc(&s.far.counters, 2 * sizeof(unsigned int)));
@@ -464,7 +463,7 @@ void Engine<T>::destroy() {
     km_free(s.C[0]); km_free(s.C[1]); km_free(s.Cd[0]); km_free(s.Cd[1]); km_free(s.cnorm); km_free(s.shift_k); km_free(s.empties);
     km_free(s.st); km_free(s.cand_val); km_free(s.cand_row); km_free(s.sum_partials);
     km_free(s.ticket); km_free(s.reloc_rec); km_free(s.reloc_all);
-    km_free(s.far.tmax); km_free(s.far.trow); km_free(s.far.cval); km_free(s.far.crow); km_free(s.far.counters);
+    km_free(s.far.tmax); km_free(s.far.cval); km_free(s.far.crow); km_free(s.far.counters);
     km_free(s.far.thr); km_free(s.far.oval); km_free(s.far.orow);
     km_free(s.shift_log); km_free(s.changed_log); km_free(s.reloc_log); km_free(s.xstat);
     PinnedWords::get().give(s.host_pin);

@@ -318,7 +318,6 @@ constexpr int kFarRank = 2048;     // values one CTA orders by counting
 constexpr int kFarDirectMax = 4;   // up to this many empty clusters are served one pass at a time
 struct FarScratch {
   double* tmax;                  // [grid * 256] thread maxima
-  unsigned long long* trow;
   double* cval;                  // [cap] candidates
   unsigned long long* crow;
   double* oval;                  // [>= E] result, descending
@@ -353,6 +352,74 @@ __device__ __forceinline__ void block_argmax(double& bv, unsigned long long& br,
   __syncthreads();
 }
 
+// The E-th largest of m values, of which negative ones do not count, or a number a little below it: for one CTA of 256
+// threads.  Non-negative doubles order as their bits, so 11 bits at a time from the top: count the values by those
+// bits among the ones that agree with the choice so far, and choose the bits that hold the E-th.  Ends early when
+// so few values reach the choice that more bits would not shorten the list of candidates.  0 if there are fewer than E.
+// hist: 2048 words of shared memory.  Bound by the reads from L2 (m / 256 per thread and round); 37,888 values, two
+// to three rounds.
+__device__ double kth_largest(const double* v, int m, int E, unsigned int* hist) {
+  __shared__ unsigned int s_wsum[8], s_bin, s_above, s_count;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  unsigned long long prefix = 0;
+  unsigned int need = (unsigned int)E, larger = 0;   // larger: values beyond the choice so far
+  for (int top = 64; top > 0; top -= 11) {
+    const int shift = top > 11 ? top - 11 : 0;
+    const unsigned int mask = (1u << (top - shift)) - 1u;
+    for (int i = tid; i < 2048; i += 256) hist[i] = 0;
+    __syncthreads();
+    for (int c0 = 0; c0 < m; c0 += 4 * 256) {
+      double x[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int c = c0 + u * 256 + tid;
+        x[u] = c < m ? __ldcg(v + c) : -1.0;
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const unsigned long long bits = (unsigned long long)__double_as_longlong(x[u]);
+        const bool in = x[u] >= 0.0 && (top == 64 || ((bits ^ prefix) >> (top & 63)) == 0);
+        const unsigned int bin = in ? (unsigned int)(bits >> shift) & mask : ~0u;
+        // most values share a few bins: one addition per bin and warp
+        const unsigned int peers = __match_any_sync(0xffffffffu, bin);
+        if (in && lane == __ffs((int)peers) - 1) atomicAdd(&hist[bin], (unsigned int)__popc(peers));
+      }
+    }
+    __syncthreads();
+    // thread t has the bins 2047 - 8 t ... 2040 - 8 t: sums from the top
+    unsigned int own = 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) own += hist[2047 - 8 * tid - i];
+    unsigned int incl = own;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned int p = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += p;
+    }
+    if (lane == 31) s_wsum[warp] = incl;
+    if (tid == 0) s_bin = ~0u;
+    __syncthreads();
+    for (int w = 0; w < warp; ++w) incl += s_wsum[w];
+    unsigned int above = incl - own;
+    if (above < need && need <= incl) {
+      int bin = 2047 - 8 * tid;
+      while (above + hist[bin] < need) above += hist[bin--];
+      s_bin = (unsigned int)bin;
+      s_above = above;
+      s_count = hist[bin];
+    }
+    __syncthreads();
+    const unsigned int bin = s_bin, ab = s_above, count = s_count;
+    __syncthreads();
+    if (bin == ~0u) return 0.0;   // (in the first round only: later ones hold the E-th value)
+    prefix |= (unsigned long long)bin << shift;
+    need -= ab;
+    larger += ab;
+    if (larger + count <= (unsigned int)E + 256u) break;
+  }
+  return __longlong_as_double((long long)prefix);
+}
+
 // Called by every thread of a cooperative grid of 256-thread CTAs.  On success oval / orow hold the
 // min(E, rows) farthest rows in descending order and *n_out their number.
 __device__ bool top_far(cg::grid_group& grid, const double* __restrict__ dist, size_t n, int E, const FarScratch& fs,
@@ -361,58 +428,18 @@ __device__ bool top_far(cg::grid_group& grid, const double* __restrict__ dist, s
   const size_t b0 = (size_t)blockIdx.x * per;
   const size_t b1 = (b0 + per < n) ? b0 + per : n;
   const size_t gtid = (size_t)blockIdx.x * 256 + threadIdx.x;
-  const int M = (int)gridDim.x * 256, MW = (int)gridDim.x * 8;
-  // The E-th largest of the maxima of disjoint sets of rows is a lower bound of the E-th largest distance.  While
-  // the empty clusters are few beside the grid's warps, the sets are those of the warps: a thousand values, of which
-  // one CTA finds the E-th by counting, for each, how many are larger.
-  const bool by_warp = E * 4 <= MW && MW <= kFarRank;
+  const int M = (int)gridDim.x * 256;
   __shared__ double s_rank[kFarRank];
   __shared__ unsigned long long s_rank_row[kFarRank];
   {
     double bv = -1.0;
-    unsigned long long br = ~0ULL;
-    for (size_t i = b0 + threadIdx.x; i < b1; i += 256) {
-      const double v = dist[i];
-      if (v > bv) { bv = v; br = i; }
-    }
-    if (by_warp) {
-      bv = warp_max(bv);
-      if ((threadIdx.x & 31) == 0) fs.tmax[gtid >> 5] = bv;
-    } else {
-      fs.tmax[gtid] = bv;
-      fs.trow[gtid] = br;
-    }
+    for (size_t i = b0 + threadIdx.x; i < b1; i += 256) bv = fmax(bv, dist[i]);
+    fs.tmax[gtid] = bv;
     if (gtid == 0) { fs.counters[0] = 0; fs.counters[1] = 0; }
   }
   grid.sync();
-  if (blockIdx.x == 0 && by_warp) {
-    for (int c = threadIdx.x; c < MW; c += 256) s_rank[c] = __ldcg(fs.tmax + c);
-    __syncthreads();
-    for (int c = threadIdx.x; c < MW; c += 256) {
-      const double v = s_rank[c];
-      int larger = 0, equal = 0;
-      for (int u = 0; u < MW; ++u) { larger += s_rank[u] > v; equal += s_rank[u] == v; }
-      if (larger < E && larger + equal >= E) *fs.thr = v < 0.0 ? 0.0 : v;   // (every writer has the same value)
-    }
-    __syncthreads();
-  } else if (blockIdx.x == 0) {
-    // E-th largest thread maximum (removing one maximum per round)
-    double T = 0.0;
-    for (int e = 0; e < E; ++e) {
-      double bv = -1.0;
-      unsigned long long br = ~0ULL;
-      int bi = -1;
-      for (int c = threadIdx.x; c < M; c += 256) {
-        const double v = __ldcg(fs.tmax + c);
-        const unsigned long long r = __ldcg(fs.trow + c);
-        if (v > bv || (v == bv && r < br)) { bv = v; br = r; bi = c; }
-      }
-      block_argmax(bv, br, bi, s_v, s_r, s_i);
-      if (bv < 0.0) { T = 0.0; break; }      // fewer than E rows: every row is a candidate
-      T = bv;
-      if (threadIdx.x == 0) fs.tmax[bi] = -3.0;
-      __syncthreads();
-    }
+  if (blockIdx.x == 0) {
+    const double T = kth_largest(fs.tmax, M, E, reinterpret_cast<unsigned int*>(s_rank));
     if (threadIdx.x == 0) *fs.thr = T;
   }
   grid.sync();

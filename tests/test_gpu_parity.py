@@ -1701,3 +1701,33 @@ def test_a_crowded_table_does_not_slow_the_next_one(eng):
             assert h.estep_info() == (5, False)
             assert _nearest_gap(X, centers.astype(dtype), h.labels()) == 0
         h.close()
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+def test_repair_of_many_clusters_does_not_depend_on_the_order_of_the_rows(eng, dtype):
+    """250 empty clusters, and 40,000 far rows in a class of their own that no centroid serves, once shuffled among the
+    others and once in one block (data sorted by class).  The same centroids either way, and the block costs no more:
+    a threshold taken from too few sets of rows would make the whole class candidates (one pass over the distances per
+    empty cluster, 20 times the time)."""
+    rng = np.random.default_rng(8)
+    n, far, d = 1_000_000, 40_000, 8
+    blobs = rng.uniform(-5, 5, (4, d))
+    X = blobs[rng.integers(0, 4, n)] + rng.standard_normal((n, d))
+    X[500_000:500_000 + far] += 60.0
+    X = X.astype(dtype)
+    C = np.concatenate([blobs, rng.uniform(900, 1000, (250, d))]).astype(dtype)
+    shuffled = rng.permutation(n)
+    out, ms = [], []
+    for rows in (X, np.ascontiguousarray(X[shuffled])):
+        h = eng.ResidentKMeans(dtype=dtype)
+        h.upload(rows)
+        best = 1e9
+        for _ in range(3):
+            h.fit(C, 1, flags=eng.FIT_NO_FINAL_ASSIGN)
+            best = min(best, h.stats()["ms_update"])
+        assert h.stats()["relocations"] == 250
+        out.append(h.centroids())
+        ms.append(best)
+        h.close()
+    assert np.array_equal(out[0], out[1])
+    assert ms[0] < 2 * ms[1] + 1.0, ms
