@@ -197,7 +197,7 @@ __device__ __forceinline__ int kpp_select(KppShared& sh, const double* wm, int m
   double excl = __shfl_up_sync(0xffffffffu, incl, 1);
   if (lane == 0) excl = 0;
   if (lane == 31) sh.warp_sum[warp] = incl;
-  if (t == 0) sh.pick = -1;
+  if (t == 0) sh.pick = 0x7fffffff;
   __syncthreads();
   if (t == 0) {
     double acc = 0;
@@ -213,7 +213,8 @@ __device__ __forceinline__ int kpp_select(KppShared& sh, const double* wm, int m
     unsigned int c[4] = {(unsigned int)step, 0u, 0u, kStreamPlusPlus};
     const uint4 r = Philox::run(make_uint4(c[0], c[1], c[2], c[3]), make_uint2((unsigned int)seed, (unsigned int)(seed >> 32)));
     const double target = u01_53(r.x, r.y) * total;
-    // the owner is the first chunk whose end sum exceeds the target
+    // The owner is the first chunk whose end sum exceeds the target.  A sum over more chunks may be smaller in its last
+    // bit (the scan adds in another order), so two chunks can find the target between their ends: the lower one has it.
     if (end > target && !(begin > target) && b < e) {
       double acc = begin;
       int pick = -1, last_pos = -1;
@@ -223,13 +224,14 @@ __device__ __forceinline__ int kpp_select(KppShared& sh, const double* wm, int m
         if (acc > target) { pick = i; break; }
       }
       if (pick < 0) pick = last_pos;
-      if (pick >= 0) sh.pick = pick;
+      if (pick >= 0) atomicMin(&sh.pick, pick);
     }
   }
   __syncthreads();
   if (t == 0) {
     int pick = sh.pick;
-    if (pick < 0) {
+    if (pick == 0x7fffffff) {
+      pick = -1;
       // zero total weight, or rounding pushed the target past the last sum
       if (total > 0) {
         for (int i = m - 1; i >= 0; --i)
