@@ -261,6 +261,7 @@ struct Engine : EngineBase {
     if (!on || d > tch::kMaxD || k <= 16 || k > tch::kMaxK) return false;
     size_t rows = 0;
     for (const auto& s : shards) rows = std::max(rows, s.rows);
+    if (rows > 0x7fffffffULL / tc::kBM * tc::kBM) return false;   // row numbers are ints there
     const double work = (double)rows * k * d;
     return std::is_same<T, float>::value ? work >= (d % 4 == 0 ? 2e9 : 5e8) : (d >= 8 && work >= 1e8);
   }

@@ -423,6 +423,7 @@ template <int P>
 inline int half_launch_p(HalfPlan& pl, tcb::BigPlan& tb, int* labels, IterState* st, bool count_changes, float tol_rel,
                          int num_sms, cudaStream_t stream) {
   const size_t n_sub = (pl.rows + kBM - 1) / kBM;
+  if (n_sub > 0x7fffffffULL / kBM) KM_FAIL(KM_EINVAL, "shard too large for the tensor-core kernel");
   const int grid = (int)std::min<size_t>(n_sub, (size_t)num_sms);
   const size_t smem = half_smem_bytes(tb.d, tb.kpad);
   KM_CUDA(allow_smem(assign_tc_half_kernel<P>, smem));
