@@ -46,22 +46,25 @@ def _check_data_content(do_check, name, data):
             raise ValueError("%s contains Inf or NaN" % name)
 
 
-def _host_check(do_check, name, data):
+def _host_check(est, name, data):
     """The part of the check above that the device does not make: float32 / float64 data is checked there (every call
     looks for the largest magnitude anyway), whole numbers are finite.  The numpy pass over a 256 MB matrix took
-    five times as long as the whole prediction."""
-    if data.dtype not in (np.float32, np.float64) and data.dtype.kind not in "iub":
-        _check_data_content(do_check, name, data)
+    five times as long as the whole prediction.  Without a device to make it, all of it is made here."""
+    if est.n_gpus == 0 or (data.dtype not in (np.float32, np.float64) and data.dtype.kind not in "iub"):
+        _check_data_content(est.do_checks, name, data)
 
 
 @contextlib.contextmanager
-def _device_check(do_check, name):
-    """The device's refusal of NaN / Inf in the data, reported as `_check_data_content` reports it."""
+def _device_check(est, name):
+    """The device's refusal of NaN / Inf in the data, reported as `_check_data_content` reports it: the estimator is as it
+    was before the call."""
     from ..libs import lib_kmeans
+    double_precision = est.double_precision
     try:
         yield
     except lib_kmeans.KMeansLibError as e:
-        if do_check == 1 and e.code == lib_kmeans.ENONFINITE and "input data" in str(e):
+        if est.do_checks == 1 and e.code == lib_kmeans.ENONFINITE and "input data" in str(e):
+            est.double_precision = double_precision
             raise ValueError("%s contains Inf or NaN" % name) from e
         raise
 
@@ -210,8 +213,8 @@ class KMeansH2O(object):
         the host or sends to scikit-learn (kmeans.py:508-521, 800-804) - go through the resident engine,
         which converts on the device and carries the weights."""
         X_np = _get_data(X)
-        _host_check(self.do_checks, "X", X_np)
-        with _device_check(self.do_checks, "X"):
+        _host_check(self, "X", X_np)
+        with _device_check(self, "X"):
             if sample_weight is not None or X_np.dtype not in (np.float32, np.float64):
                 self._fit_resident(X_np, sample_weight)
             else:
@@ -325,15 +328,15 @@ class KMeansH2O(object):
         lib = self._load_lib()
         X_np = _get_data(X)
         cols, rows = self._validate_centroids(X_np)
-        _host_check(self.do_checks, "X", X_np)
+        _host_check(self, "X", X_np)
         if X_np.dtype not in (np.float32, np.float64):
             return self._resident_apply(X_np, "predict")
-        c_X = self._toc(X_np)
-        dtype = np.float64 if self.double_precision else np.float32
-        centers = np.ascontiguousarray(self.cluster_centers_, dtype=dtype).reshape(-1)
-        c_res = np.zeros(rows, np.int32)
-        fn = lib.make_ptr_double_kmeans if self.double_precision else lib.make_ptr_float_kmeans
-        with _device_check(self.do_checks, "X"):
+        with _device_check(self, "X"):
+            c_X = self._toc(X_np)
+            dtype = np.float64 if self.double_precision else np.float32
+            centers = np.ascontiguousarray(self.cluster_centers_, dtype=dtype).reshape(-1)
+            c_res = np.zeros(rows, np.int32)
+            fn = lib.make_ptr_double_kmeans if self.double_precision else lib.make_ptr_float_kmeans
             fn(1, self.verbose, self.random_state, self._gpu_id, self.n_gpus, rows, cols,
                self.cluster_centers_.shape[0], self._max_iter, 0, self.tol, c_X, centers,
                np.empty([], dtype), c_res)

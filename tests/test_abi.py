@@ -72,3 +72,18 @@ def test_wrapper_cpu_backend_and_params():
         est.set_params(bogus=1)
     with pytest.raises(ValueError):
         h2o4gpu_b200.KMeansH2O(init="nonsense")
+
+
+def test_non_finite_data_is_refused_without_a_gpu_too():
+    """n_gpus = 0 (or a machine without one): no device looks at the data, so the wrapper does, before it asks for one."""
+    import pytest
+    import h2o4gpu_b200
+    X = np.ones((6, 2))
+    X[3, 1] = np.inf
+    for dtype in (np.float32, np.float64):
+        est = h2o4gpu_b200.KMeansH2O(n_clusters=2, n_gpus=0)
+        with pytest.raises(ValueError, match="contains Inf or NaN"):
+            est.fit(X.astype(dtype))
+        est.cluster_centers_ = X[:2].copy()
+        with pytest.raises(ValueError, match="contains Inf or NaN"):
+            est.predict(X.astype(dtype))

@@ -1732,3 +1732,21 @@ def test_repair_of_many_clusters_does_not_depend_on_the_order_of_the_rows(eng, d
         h.close()
     assert np.array_equal(out[0], out[1])
     assert ms[0] < 2 * ms[1] + 1.0, ms
+
+
+@pytest.mark.parametrize("first,second", [(np.float32, np.float64), (np.float64, np.float32)])
+def test_a_refused_matrix_leaves_the_estimator_as_it_was(built_lib, first, second):
+    """fit and predict refuse NaN in a matrix of the other precision: the fitted model still predicts integers, whose
+    precision is the model's, as it did."""
+    from h2o4gpu_b200 import KMeansH2O
+    rng = np.random.default_rng(4)
+    X = rng.integers(0, 50, (1000, 6))
+    m = KMeansH2O(n_clusters=4, max_iter=5, random_state=1).fit(X.astype(first))
+    want, precision, centers = m.predict(X), m.double_precision, m.cluster_centers_.copy()
+    bad = X.astype(second)
+    bad[10, 2] = np.nan
+    for call in (lambda: m.fit(bad), lambda: m.fit(bad, sample_weight=np.ones(1000)), lambda: m.predict(bad)):
+        with pytest.raises(ValueError, match="contains Inf or NaN"):
+            call()
+        assert m.double_precision == precision == int(first == np.float64)
+        assert np.array_equal(m.cluster_centers_, centers) and np.array_equal(m.predict(X), want)
