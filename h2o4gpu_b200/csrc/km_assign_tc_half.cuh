@@ -165,8 +165,11 @@ assign_tc_half_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
                       size_t n, int n_sub, int kpad, int ksteps, IterState* st, int count_changes,
                       uint4* __restrict__ cand_near, unsigned int cand_cap,
                       unsigned int all_limit, float tol_rel, float tol_floor, float sx, float sxsb,
-                      unsigned int wait_iters) {
-  if (st->full_rows) return;   // this matrix left too many rows open before: the kernel behind this one has the pass
+                      unsigned int wait_iters, unsigned int* host_whole) {
+  if (st->full_rows) {   // this matrix left too many rows open before: the kernel behind this one has the pass
+    if (host_whole && blockIdx.x == 0 && threadIdx.x == 0) *host_whole = 1;
+    return;
+  }
   constexpr int NX = x_stages(P), NB = b_stages(P);
   constexpr uint32_t kXBytes = P * kPanel;
   constexpr uint32_t kAccCol = 2u * P * 32u;     // accumulators behind the two A buffers
@@ -486,10 +489,12 @@ assign_tc_half_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
       st->half_done = 0;
       const unsigned int cand = atomicAdd(&st->cand_count, 0u), all = atomicAdd(&st->cand_all, 0u);
       st->cand_all = 0;
-      if (cand > cand_cap || all > all_limit) {
+      const bool whole = cand > cand_cap || all > all_limit;
+      if (whole) {
         st->full_rows = 1;
         st->cand_count = 0;
       }
+      if (host_whole) *host_whole = whole ? 1 : 0;
     }
   }
   if (warp == 1) {

@@ -220,7 +220,9 @@ struct Engine : EngineBase {
   int check_data();
   int set_centroids(int k_, const T* host_c);
   int fit(int k_, int max_iter, double threshold, const T* init, int flags);
-  int assign_all(int flags);
+  int assign_all(int flags, bool closes_fit = false);
+  // waits for passes with nothing queued behind them and makes them again on whole rows if need be (*again)
+  int settle_alone(bool* again = nullptr);
   int transform_shard(int local, T* out_host, size_t ld);
   int inertia(double* out);
   int inertia_launch();
@@ -231,7 +233,8 @@ struct Engine : EngineBase {
   SplitTable split_table(Shard<T>& s, bool use_tc);
   int launch_close(Shard<T>& s, int run_if, int it, double inv, bool use_tc);
   int poll_seq = 0;   // sequence number the finalize kernels publish to pinned memory
-  bool tc_ok(int flags) const;
+  // single: for one label pass
+  bool tc_ok(int flags, bool single = false) const;
   // which tensor-core distance kernel labels this shape: 1 table resident (d 32/64, k <= 128), 2 table streamed
   // (d <= 256), 3 few centroids and wide rows, 4 both operands streamed (wider rows, many centroids), 5 float64 rows
   // rounded to fp16, 0 none
@@ -290,20 +293,34 @@ struct Engine : EngineBase {
   int stream_refresh(Shard<T>& s, const OutRule& rule);   // operand table and plan of the streaming kernel for the current centroids
   // split the current centroids for the tensor-core kernel; for labels the table leaves out those that no row can be
   // nearest to
-  int tc_refresh(Shard<T>& s, bool for_labels = true);
+  // What the refresh prepares: the E-steps of a fit, which the host queues ahead; one label pass that the host waits for;
+  // that pass once more on whole rows, because the rounded ones left too many open.
+  enum class Pass { fit, single, whole };
+  int tc_refresh(Shard<T>& s, Pass pass, bool for_labels = true);
   int launch_assign(Shard<T>& s, bool use_tc, bool count_changes);
-  tc::SplitBuild tc_split_build = tc::SplitBuild::no;   // whether the running fit pays for the split copy of X
-  // Begins a call that labels rows.  The caller may have written other values into a matrix it lends
-  // (attach_device) since the last call, so the rounded rows are made from what is there now: they live as long as one
-  // call.  Only the split copy of a long fit stays, as it always did, and what was taken when the matrix was
-  // attached (max |x|, row norms, padded rows).  A matrix this handle uploaded cannot change under it.
+  bool tc_split_build = false;   // the running fit has enough iterations to pay for the split copy of X
+  // A matrix the caller lends (attach_device) may hold other values at the next call.  Rows that the kernels used to read
+  // anew in every pass are therefore rounded anew by every call; what was always taken once per attachment stays (max
+  // |x|, row norms, the copies of rows that are not 16-byte aligned and of long fits at 64 columns).  A matrix this
+  // handle uploaded cannot change under it.
+  bool lent() const { return !shards.empty() && shards[0].X != shards[0].X_owned; }
   void drop_row_copies() {
-    for (auto& s : shards) {
-      if (s.X == s.X_owned) continue;
-      s.tchp.of = nullptr;
-      if (!s.tcp.xsplit_kept) s.tcp.xsplit_of = nullptr;
-    }
+    if (lent() && (std::is_same<T, double>::value || d % 4 == 0))
+      for (auto& s : shards) s.tchp.of = nullptr;
   }
+  // Whether rounding the rows pays for `passes` label passes.  Float32 rows of a lent matrix: rounding takes about 1.6 ps
+  // per element, the one-product kernel saves 2.5 fs per element and centroid (500,000 x 128 and 1e6 x 64 rows).
+  // Float64 rows in a single pass: the float64 matrix unit takes 0.069 ps per product, 5e8 of them what the four
+  // further launches and the rounding do (60,000 x 40, 50 centroids: 101 us a call against 118; 200,000 x 64, 100
+  // centroids: 240 against 170); without the unit (odd widths) the FP64 pipe is behind earlier.
+  bool rounding_pays(int passes) const {
+    if (std::is_same<T, float>::value) return d % 4 != 0 || !lent() || (double)passes * k >= 640.0;
+    if (passes > 1 || d % 2 != 0 || k <= 32) return true;
+    size_t rows = 0;
+    for (const auto& s : shards) rows = std::max(rows, s.rows);
+    return (double)rows * k * d >= 5e8;
+  }
+  int fit_passes = 1;   // label passes of the running fit
   double xmax_all() const {
     double m = 0;
     for (const auto& s : shards) m = std::max(m, s.xmax);
@@ -492,7 +509,6 @@ int Engine<T>::attach_device(int local, const T* dX, size_t rows, size_t cols, s
   // even when the new one has the same address and shape
   s.tcp.xnorm_of = nullptr;
   s.tcp.xsplit_of = nullptr;
-  s.tcp.xsplit_kept = false;
   s.tcp.ready = false;
   s.tcbp.ready = false;
   s.tchp.of = nullptr;
@@ -1108,9 +1124,7 @@ int Engine<T>::set_centroids(int k_, const T* host_c) {
   for (auto& s : shards) {
     DevGuard g(s.dev);
     KM_CUDA(cudaMemcpyAsync(s.C[0], host_c, (size_t)k * d * sizeof(T), cudaMemcpyHostToDevice, s.stream));
-    // another table may be less crowded than the one that sent the E-step on to whole rows
-    KM_CUDA(cudaMemsetAsync(&s.st->full_rows, 0, sizeof(unsigned int), s.stream));
-    cnorm_kernel<T><<<k, 128, 0, s.stream>>>(s.C[0], k, d, s.cnorm, s.Cd[0]);
+    cnorm_kernel<T><<<k, 128, 0, s.stream>>>(s.C[0], k, d, s.cnorm, s.Cd[0], s.st);
     KM_CUDA(cudaGetLastError());
     ++launches;
     // host_c may be freed by the caller right after this returns
@@ -1340,7 +1354,7 @@ int Engine<T>::launch_accumulate(Shard<T>& s, T scale, long long* dst, const uns
 // The tcgen05 kernel serves float32 shards with d in {32, 64} and 16 < k <= 128 on
 // compute capability 10.x; everything else runs on the SIMT kernels.
 template <typename T>
-bool Engine<T>::tc_ok(int flags) const {
+bool Engine<T>::tc_ok(int flags, bool single) const {
   if (flags & KM_FIT_FORCE_SIMT) return false;
   const int kind = tc_kind();
   if (kind == 0) return false;
@@ -1349,12 +1363,14 @@ bool Engine<T>::tc_ok(int flags) const {
     if (kind == 5) continue;
     if (d % 4 == 0) {
       if ((reinterpret_cast<uintptr_t>(s.X) & 15) != 0) return false;
+    } else if (single && half_shape_ok() && s.tchp.holds(s.rows, d)) {
+      continue;   // it needs no padded copy, and asking for the free memory takes 60 us
     } else if (!(s.xpad && s.xpad_cap >= s.rows * (size_t)dtc())) {
       // the padded copy must fit beside the shard (with room to spare for the fit's own buffers)
       size_t free_b = 0, total_b = 0;
       DevGuard g(s.dev);
       if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return false;
-      if (free_b < s.rows * (size_t)dtc() * sizeof(T) + ((size_t)1 << 30)) return false;
+      if (free_b + s.tchp.bytes() < s.rows * (size_t)dtc() * sizeof(T) + ((size_t)1 << 30)) return false;
     }
   }
   double xmax = 0;
@@ -1364,10 +1380,11 @@ bool Engine<T>::tc_ok(int flags) const {
 }
 
 template <typename T>
-int Engine<T>::tc_refresh(Shard<T>& s, bool for_labels) {
+int Engine<T>::tc_refresh(Shard<T>& s, Pass pass, bool for_labels) {
   const OutRule rule = for_labels ? out_rule(xmax_all(), d) : OutRule{};
-  const bool half = half_shape_ok() && (tc_kind() == 2 || tc_kind() == 5);
-  s.tchp.on = false;
+  const bool half = pass != Pass::whole && half_shape_ok() && (tc_kind() == 2 || tc_kind() == 5) &&
+                    rounding_pays(pass == Pass::fit ? fit_passes : 1);
+  s.tchp.on = s.tchp.alone = false;
   if constexpr (std::is_same<T, double>::value) {
     double xmax = 0;
     for (const auto& sh : shards) xmax = std::max(xmax, sh.xmax);
@@ -1385,10 +1402,32 @@ int Engine<T>::tc_refresh(Shard<T>& s, bool for_labels) {
     if (!tc::pick_scales(xmax, std::max(xmax, cbound), &tc_sx, &tc_sb))
       KM_FAIL(KM_EINVAL, "data magnitude outside the range of the tensor-core kernel");
     if (s.rows > 0xffffffffULL) KM_FAIL(KM_EINVAL, "shard too large for the tensor-core kernel");
-    KM_TRY(ensure_amb(s, tc_kind() == 1));
     const int kind = tc_kind();
+    if (half && pass == Pass::single && d % 4 != 0 && s.xpad_of != s.X) {
+      // Rows that are not 16-byte aligned: the padded copy (as large as the matrix), the list of rows and the norms serve
+      // only the kernel behind.  A call that waits for its one pass makes them when it comes to that (1e6 x 50 rows:
+      // 216 MB less to allocate for a new matrix).
+      KM_TRY(tcb::big_tables(s.tcbp, k, d, true));
+      s.tchp.on = s.tchp.alone = tch::half_rows<T>(s.tchp, s.X, s.rows, d, tc_sx, s.num_sms, s.stream, &launches);
+      if (s.tchp.alone) {
+        s.tcbp.sx = tc_sx;
+        s.tcbp.sb = tc_sb;
+        KM_TRY(tcb::big_prep(s.tcbp, s.C[cur], s.cnorm, rule, s.stream));
+        ++launches;
+        return KM_OK;
+      }
+    }
+    KM_TRY(ensure_amb(s, kind == 1));
     // what the call cannot do without comes before the rounded rows: tc_ok() has seen that it fits
-    if (d % 4 != 0) KM_TRY(ensure_xpad(s, !half));
+    if (d % 4 != 0) {
+      int rc = ensure_xpad(s, !half);
+      if (rc != KM_OK && s.tchp.xh) {   // rounded rows of an earlier single pass are in the way
+        cudaGetLastError();
+        s.tchp.release();
+        rc = ensure_xpad(s, !half);
+      }
+      KM_TRY(rc);
+    }
     if (half) {
       KM_TRY(tcb::big_tables(s.tcbp, k, d, true));
       s.tchp.on = tch::half_rows<T>(s.tchp, s.X, s.rows, d, tc_sx, s.num_sms, s.stream, &launches);
@@ -1490,6 +1529,7 @@ int Engine<T>::launch_assign(Shard<T>& s, bool use_tc, bool count_changes) {
       const bool half = s.tchp.on;
       if (half) {
         KM_TRY(launch_half(s, count_changes));
+        if (s.tchp.alone) return KM_OK;   // the caller looks whether whole rows are needed
         // behind it, gated on the device, the pass that needs no list of open rows
         if (d % 4 != 0 && s.xpad_of != s.X) {
           pad_rows_kernel<T><<<s.num_sms * 16, 256, 0, s.stream>>>(s.X, s.rows, d, dtc(), s.xpad, s.st);
@@ -1561,7 +1601,8 @@ int Engine<T>::launch_assign(Shard<T>& s, bool use_tc, bool count_changes) {
 // the one-product kernel and the exact pass over the rows it leaves open
 template <typename T>
 int Engine<T>::launch_half(Shard<T>& s, bool count_changes) {
-  KM_TRY(tch::half_launch(s.tchp, s.tcbp, s.labels, s.st, count_changes, tc::tol_rel_of(d), s.num_sms, s.stream));
+  KM_TRY(tch::half_launch(s.tchp, s.tcbp, s.labels, s.st, count_changes, tc::tol_rel_of(d), s.num_sms, s.stream,
+                          s.tchp.alone ? reinterpret_cast<unsigned int*>(&s.host_pin[4]) : nullptr));
   const int grid = s.num_sms * 8, threads = tch::kExactWarps * 32, cc = count_changes ? 1 : 0;
   if constexpr (std::is_same<T, double>::value) {
     tch::half_exact_f64_kernel<<<grid, threads, 0, s.stream>>>(s.X, d, s.C[cur], k, s.tcbp.kpad, s.tchp.cand_near, s.st,

@@ -62,7 +62,8 @@ absmax_kernel(const T* __restrict__ X, size_t count, double* __restrict__ out_ma
 // ---- |c|^2 of a centroid table -------------------------------------------------
 template <typename T>
 __global__ void __launch_bounds__(128)
-cnorm_kernel(const T* __restrict__ C, int k, int d, T* __restrict__ cnorm, double* __restrict__ C_double = nullptr) {
+cnorm_kernel(const T* __restrict__ C, int k, int d, T* __restrict__ cnorm, double* __restrict__ C_double,
+             IterState* st) {
   __shared__ double red[4];
   int j = blockIdx.x;
   double s = 0;
@@ -75,6 +76,8 @@ cnorm_kernel(const T* __restrict__ C, int k, int d, T* __restrict__ cnorm, doubl
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
   __syncthreads();
   if (threadIdx.x == 0) cnorm[j] = (T)(red[0] + red[1] + red[2] + red[3]);
+  // another table may be less crowded than the one that sent the E-step on to whole rows
+  if (j == 0 && threadIdx.x == 0) st->full_rows = 0;
 }
 
 // ---- per-iteration bookkeeping: empties, largest cluster ----------------------

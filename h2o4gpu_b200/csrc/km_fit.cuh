@@ -40,7 +40,7 @@ static int ensure_logs(Shard<T>& s, int n) {
 // E-step on every local shard with the current centroids (final pass of fit,
 // predict).  Labels change counters are not touched.
 template <typename T>
-int Engine<T>::assign_all(int flags) {
+int Engine<T>::assign_all(int flags, bool closes_fit) {
   TraceRange trace_range("kmeans.assign");
   if (!have_centroids) KM_FAIL(KM_ESTATE, "no centroids set");
   for (auto& s : shards) {
@@ -48,12 +48,31 @@ int Engine<T>::assign_all(int flags) {
     DevGuard g(s.dev);
     // the same dispatch as the E-step of a fit (launch_assign picks the streaming kernel for few
     // centroids and wide rows, the small-k kernel for narrow ones)
-    const bool use_tc = tc_ok(flags) && (!smallk_ok(false) || tc_kind() == 3);
+    const bool use_tc = tc_ok(flags, !closes_fit) && (!smallk_ok(false) || tc_kind() == 3);
     if (use_tc) {
-      KM_TRY(tc_refresh(s));
+      KM_TRY(tc_refresh(s, closes_fit ? Pass::fit : Pass::single));
       KM_CUDA(cudaMemsetAsync(&s.st->amb_count, 0, 2 * sizeof(unsigned int), s.stream));   // and cand_count
     }
     KM_TRY(launch_assign(s, use_tc, false));
+  }
+  return KM_OK;
+}
+
+template <typename T>
+int Engine<T>::settle_alone(bool* again) {
+  for (auto& s : shards) {
+    if (!s.tchp.alone) continue;
+    s.tchp.alone = false;
+    DevGuard g(s.dev);
+    KM_CUDA(cudaStreamSynchronize(s.stream));
+    if (*reinterpret_cast<volatile unsigned int*>(&s.host_pin[4]) == 0) continue;
+    if (again) *again = true;
+    int rc = tc_refresh(s, Pass::whole);
+    const bool full = rc == KM_ENOMEM;   // no memory for the padded copy: the kernels that need none
+    if (full) { cudaGetLastError(); rc = KM_OK; }
+    KM_TRY(rc);
+    KM_TRY(launch_assign(s, !full, false));
+    s.estep_kernel = 5;   // (sent on)
   }
   return KM_OK;
 }
@@ -188,11 +207,11 @@ int Engine<T>::fit(int k_, int max_iter, double threshold, const T* init, int fl
   const bool fused = smallk_ok(true) && !(flags & KM_FIT_FORCE_SPLIT) && !weighted;
   const bool use_tc = !fused && tc_ok(flags);
   // the fp16 copy of X (d = 64 tensor-core kernel without converter warps) takes the place of the row norms'
-  // pass and costs about as much more as one iteration saves
-  tc_split_build = (max_iter >= 16 || (flags & KM_FIT_PRESPLIT)) ? tc::SplitBuild::keep
-                   : max_iter >= 3                               ? tc::SplitBuild::call
-                                                                 : tc::SplitBuild::no;
-  struct SplitBuildGuard { tc::SplitBuild& f; ~SplitBuildGuard() { f = tc::SplitBuild::no; } } split_build_guard{tc_split_build};
+  // pass and costs about as much more as one iteration saves.  Of a lent matrix it would have to be made by every
+  // such fit, where the norms are there already: only long fits do, and keep it
+  tc_split_build = max_iter >= (lent() ? 16 : 3) || (flags & KM_FIT_PRESPLIT);
+  struct SplitBuildGuard { bool& f; ~SplitBuildGuard() { f = false; } } split_build_guard{tc_split_build};
+  fit_passes = max_iter + ((flags & KM_FIT_NO_FINAL_ASSIGN) ? 0 : 1);
   // incremental M-step (km_accumulate_delta.cuh): on unless the caller or the environment asks
   // for a full recomputation every iteration; a shard switches to it, on the device, in the
   // iterations where at most 1/8 of its labels moved (kDeltaFraction)
@@ -238,7 +257,7 @@ int Engine<T>::fit(int k_, int max_iter, double threshold, const T* init, int fl
     s.moved_bits_valid = false;
     if (s.pflush)   // all zero between iterations; cleared here in case an earlier fit stopped half-way
       KM_CUDA(cudaMemsetAsync(s.pflush, 0, s.gacc_count(k, d) * kFlushPad * sizeof(long long), s.stream));
-    if (use_tc) KM_TRY(tc_refresh(s));
+    if (use_tc) KM_TRY(tc_refresh(s, Pass::fit));
   }
 
   // events on shard 0: [4*it + 0..3] = start, after E-step, after sums, after close
@@ -391,7 +410,7 @@ int Engine<T>::fit(int k_, int max_iter, double threshold, const T* init, int fl
     cudaEventRecord(ev[ev.size() - 2], s0.stream);
   }
   if (!(flags & KM_FIT_NO_FINAL_ASSIGN)) {
-    rc = assign_all(flags);
+    rc = assign_all(flags, true);
     if (rc != KM_OK) { free_events(); return rc; }
   }
   {
@@ -559,11 +578,11 @@ int Engine<T>::transform_shard(int local, T* out_host, size_t ld) {
     // tensor-core kernels with a store epilogue (they need max|x| for the operand scales, i.e. a checked
     // matrix): the wide-row kernel for few centroids, the kernel that streams both operands for the rest
     if (tc_kind() == 3 && tc_ok(0)) {
-      rc = tc_refresh(s, false);
+      rc = tc_refresh(s, Pass::single, false);
       wide = rc == KM_OK;
     } else if (tcs::stream_shape_ok(k, dtc()) && tc_ok(0)) {
       if (tc_kind() == 4) {
-        rc = tc_refresh(s, false);
+        rc = tc_refresh(s, Pass::single, false);
       } else {
         // the shape's own labelling kernel keeps its plan; the streaming kernel gets one beside it
         double xmax = 0;

@@ -389,6 +389,7 @@ int init_centroids(Engine<T>& e, int k, int seed, int method, std::vector<T>* ou
     if (m_new > 0) {
       rc = e.set_centroids(m_new, fresh.data());
       if (rc == KM_OK) rc = e.assign_all(0);
+      if (rc == KM_OK) rc = e.settle_alone();
       if (rc != KM_OK) break;
       for (auto& s : e.shards) {
         DevGuard g(s.dev);
@@ -488,6 +489,7 @@ int init_centroids(Engine<T>& e, int k, int seed, int method, std::vector<T>* ou
   // 3. weights = rows (sample weight) nearest to each candidate, then weighted k-means++ on the device
   KM_TRY(e.set_centroids(m, all.data()));
   KM_TRY(e.assign_all(0));
+  KM_TRY(e.settle_alone());
   std::vector<double> w(m, 0.0);
   {
     std::vector<unsigned long long> cnt(m);

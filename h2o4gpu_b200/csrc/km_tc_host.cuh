@@ -63,7 +63,6 @@ struct Plan {
   const float* xsplit_of = nullptr;
   size_t xsplit_rows = 0;
   float xsplit_sx = 0.f;
-  bool xsplit_kept = false;     // made by a long fit (or on request): good until other data is attached
   bool xsplit_failed = false;   // no memory for it: stay with the converting kernel
   CUtensorMap tmXh;
 
@@ -114,7 +113,6 @@ inline int ensure_xnorm(Plan& pl, const float* X, size_t rows, int d, int num_sm
 
 // The fp16 copy of X for the kernel variant without converter warps (d = 64): made when the
 // matrix, its size or the scale changed; costs one pass over X and half as much memory again.
-enum class SplitBuild { no, call, keep };   // not at all, for the running call, until other data is attached
 inline bool presplit_enabled() {
   static const bool on = [] {
     const char* e = std::getenv("H2O4GPU_KM_TC_PRESPLIT");
@@ -123,13 +121,10 @@ inline bool presplit_enabled() {
   return on;
 }
 inline bool ensure_xsplit(Plan& pl, const float* X, size_t rows, int d, float sx, int num_sms, cudaStream_t stream,
-                          SplitBuild build) {
+                          bool allow_build) {
   if (d != 64 || !presplit_enabled() || pl.xsplit_failed) return false;
-  if (pl.xsplit && pl.xsplit_of == X && pl.xsplit_rows == rows && pl.xsplit_sx == sx) {
-    pl.xsplit_kept = pl.xsplit_kept || build == SplitBuild::keep;
-    return true;
-  }
-  if (build == SplitBuild::no) return false;   // a single pass (predict) does not pay for the split
+  if (pl.xsplit && pl.xsplit_of == X && pl.xsplit_rows == rows && pl.xsplit_sx == sx) return true;
+  if (!allow_build) return false;   // a single pass (predict) does not pay for the split
   if (pl.xsplit_cap < rows) {
     km_free(pl.xsplit);
     km_free(pl.xrowq);
@@ -156,7 +151,6 @@ inline bool ensure_xsplit(Plan& pl, const float* X, size_t rows, int d, float sx
   pl.xsplit_of = X;
   pl.xsplit_rows = rows;
   pl.xsplit_sx = sx;
-  pl.xsplit_kept = build == SplitBuild::keep;
   return true;
 }
 
@@ -215,12 +209,12 @@ inline float tol_floor_of(int d) { return 1.1920928955078125e-07f * std::sqrt((f
 
 inline int launch(Plan& pl, int* labels, IterState* st, bool count_changes, unsigned int* amb_rows,
                   unsigned int* amb_seg, float tol_rel, int num_sms, cudaStream_t stream, unsigned int* moved_bits,
-                  uint4* amb_near, SplitBuild split_build, int* launches) {
+                  uint4* amb_near, bool allow_split_build, int* launches) {
   const size_t tiles = (pl.x_rows + kBM - 1) / kBM;
   if (tiles > 0x7fffffffULL / kBM) KM_FAIL(KM_EINVAL, "shard too large for the tensor-core kernel");
   const int grid = (int)std::min<size_t>(tiles, (size_t)num_sms);
   const unsigned int seg_cap = (unsigned int)amb_seg_rows(pl.x_rows, num_sms);
-  const bool pre = ensure_xsplit(pl, pl.x_base, pl.x_rows, pl.d, pl.sx, num_sms, stream, split_build);
+  const bool pre = ensure_xsplit(pl, pl.x_base, pl.x_rows, pl.d, pl.sx, num_sms, stream, allow_split_build);
   if (!pre) KM_TRY(ensure_xnorm(pl, pl.x_base, pl.x_rows, pl.d, num_sms, stream));
   auto go = [&](auto fn, const CUtensorMap& tmX, bool p) -> int {
     KM_CUDA(allow_smem(fn, smem_bytes(pl.d, pl.npad, p)));
@@ -360,6 +354,14 @@ struct HalfPlan {
   uint4* cand_near = nullptr;
   unsigned int cand_cap = 0;
   bool on = false;                // the current E-steps run on the rounded rows
+  bool alone = false;             // ... with nothing queued behind them (a single pass over unaligned rows)
+
+  // a quarter of the rows: settling an open row costs about twice its share of the pass that needs no list
+  static size_t list_rows(size_t rows) { return std::max<size_t>(rows / 4, std::min<size_t>(rows, 4096)); }
+  bool holds(size_t rows, int d) const {
+    return xh_cap >= rows * (size_t)((d + 7) / 8 * 8) && rowq_cap >= rows && cand_cap >= list_rows(rows);
+  }
+  size_t bytes() const { return xh_cap * sizeof(__half) + rowq_cap * sizeof(float2) + cand_cap * sizeof(uint4); }
 
   void release() {
     km_free(xh); km_free(rowq); km_free(cand_near);
@@ -367,7 +369,7 @@ struct HalfPlan {
     xh_cap = rowq_cap = 0;
     cand_cap = 0;
     of = nullptr;
-    on = false;
+    on = alone = false;
   }
 };
 
@@ -388,10 +390,8 @@ template <typename T>
 inline bool half_rows(HalfPlan& pl, const T* X, size_t rows, int d, float sx, int num_sms, cudaStream_t stream,
                       int* launches) {
   const int ldh = (d + 7) / 8 * 8;
-  // a quarter of the rows: settling an open row costs about twice its share of the pass that needs no list
-  const size_t cap = std::max<size_t>(rows / 4, std::min<size_t>(rows, 4096));
-  const size_t elems = rows * (size_t)ldh;
-  if (pl.cand_cap < cap || pl.xh_cap < elems || pl.rowq_cap < rows) {
+  const size_t cap = HalfPlan::list_rows(rows), elems = rows * (size_t)ldh;
+  if (!pl.holds(rows, d)) {
     size_t have = pl.cand_cap;
     pl.of = nullptr;
     if (!km_room_for(elems * sizeof(__half) + rows * sizeof(float2) + cap * sizeof(uint4)) ||
@@ -421,7 +421,7 @@ inline bool half_rows(HalfPlan& pl, const T* X, size_t rows, int d, float sx, in
 
 template <int P>
 inline int half_launch_p(HalfPlan& pl, tcb::BigPlan& tb, int* labels, IterState* st, bool count_changes, float tol_rel,
-                         int num_sms, cudaStream_t stream) {
+                         int num_sms, cudaStream_t stream, unsigned int* host_whole) {
   const size_t n_sub = (pl.rows + kBM - 1) / kBM;
   if (n_sub > 0x7fffffffULL / kBM) KM_FAIL(KM_EINVAL, "shard too large for the tensor-core kernel");
   const int grid = (int)std::min<size_t>(n_sub, (size_t)num_sms);
@@ -433,18 +433,19 @@ inline int half_launch_p(HalfPlan& pl, tcb::BigPlan& tb, int* labels, IterState*
   assign_tc_half_kernel<P><<<grid, kHalfThreads, smem, stream>>>(
       pl.tmX, tb.tmBhi, tb.cn, pl.rowq, labels, pl.rows, (int)n_sub, tb.kpad, (tb.d + 15) / 16, st,
       count_changes ? 1 : 0, pl.cand_near, pl.cand_cap, all_limit, tol_rel, tc::tol_floor_of(tb.d),
-      tb.sx, tb.sx * tb.sb, wait_limits().mbar_iters);
+      tb.sx, tb.sx * tb.sb, wait_limits().mbar_iters, host_whole);
   KM_CUDA(cudaGetLastError());
   return KM_OK;
 }
 
+// host_whole (or null): pinned word that receives st->full_rows as the kernel leaves it
 inline int half_launch(HalfPlan& pl, tcb::BigPlan& tb, int* labels, IterState* st, bool count_changes, float tol_rel,
-                       int num_sms, cudaStream_t stream) {
+                       int num_sms, cudaStream_t stream, unsigned int* host_whole) {
   switch (panels_of(tb.d)) {
-    case 1: return half_launch_p<1>(pl, tb, labels, st, count_changes, tol_rel, num_sms, stream);
-    case 2: return half_launch_p<2>(pl, tb, labels, st, count_changes, tol_rel, num_sms, stream);
-    case 3: return half_launch_p<3>(pl, tb, labels, st, count_changes, tol_rel, num_sms, stream);
-    default: return half_launch_p<4>(pl, tb, labels, st, count_changes, tol_rel, num_sms, stream);
+    case 1: return half_launch_p<1>(pl, tb, labels, st, count_changes, tol_rel, num_sms, stream, host_whole);
+    case 2: return half_launch_p<2>(pl, tb, labels, st, count_changes, tol_rel, num_sms, stream, host_whole);
+    case 3: return half_launch_p<3>(pl, tb, labels, st, count_changes, tol_rel, num_sms, stream, host_whole);
+    default: return half_launch_p<4>(pl, tb, labels, st, count_changes, tol_rel, num_sms, stream, host_whole);
   }
 }
 

@@ -202,6 +202,7 @@ int predict_impl(int verbose, int gpu_id, int n_gpu, size_t rows, size_t cols, i
   KM_TRY(e->check_data());
   KM_TRY(e->set_centroids(k, centroids));
   KM_TRY(e->assign_all(0));
+  KM_TRY(e->settle_alone());
   bool a = false;
   KM_TRY(out_buffer(pred_labels, rows, &a));
   size_t off = 0;
@@ -319,10 +320,14 @@ static int assign_sync(km::Engine<T>* e) {
     cudaEventRecord(e0, e->shards[0].stream);
   }
   int rc = e->assign_all(0);
-  {
+  auto pass_ends = [&]() {
     km::DevGuard g(e->shards[0].dev);
     cudaEventRecord(e1, e->shards[0].stream);
-  }
+  };
+  pass_ends();
+  bool again = false;
+  if (rc == KM_OK) rc = e->settle_alone(&again);
+  if (again) pass_ends();
   for (auto& s : e->shards) {
     km::DevGuard g(s.dev);
     cudaError_t ce = cudaStreamSynchronize(s.stream);

@@ -134,9 +134,9 @@ int kmeans_nccl_unique_id(void* out128);
 /* Attach a shard that already lives on local device `local` (borrowed pointer,
  * row-major rows x cols, 16-byte aligned).  n_total = rows over all ranks.  The shard
  * should keep its values while it is attached; attach it again after changing them: max |x|,
- * the check for NaN / Inf, row norms, padded rows and the rounded rows of a long fit (16
- * iterations, or KM_FIT_PRESPLIT, at 64 columns) are taken once per attachment.  The rows
- * themselves are read anew by every call. */
+ * the check for NaN / Inf, row norms and, for labels, the copies of float32 rows whose width is
+ * not a multiple of four and of a long fit (16 iterations, or KM_FIT_PRESPLIT) at 64 columns are
+ * taken once per attachment.  Other rows are read anew by every call. */
 int kmeans_attach_device(kmeans_handle_t h, int local, const void* dX, size_t rows, size_t cols,
                          size_t n_total);
 /* Upload a host matrix: rows are split contiguously over the local devices
@@ -180,9 +180,9 @@ int kmeans_set_sample_weight(kmeans_handle_t h, const void* weights, size_t coun
 #define KM_FIT_FULL_SUMS 16       /* recompute the centroid sums from every row in every
                                   * iteration (default: exact incremental update once few
                                   * labels change; same bits either way)              */
-#define KM_FIT_PRESPLIT 32        /* d = 64 tensor-core path: round the rows to fp16 whatever the iteration count (by
-                                    default fits of three iterations or more do) and keep the rounded rows until other
-                                    data is attached (by default after 16 iterations or more) */
+#define KM_FIT_PRESPLIT 32        /* d = 64 tensor-core path: round the rows to fp16 whatever the iteration count
+                                    and keep them until other data is attached (by default fits of 16 iterations or
+                                    more do, of three or more on an uploaded matrix) */
 
 /* Lloyd iterations on the resident shards from k x cols host centroids.
  * Stops after max_iter, or earlier when threshold > 0 and the summed squared

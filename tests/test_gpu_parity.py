@@ -1519,10 +1519,11 @@ def test_narrow_rows_labels(eng, dtype, n, d, k):
 
 # ---- a lent matrix that changes between calls ------------------------------------------------------
 @pytest.mark.parametrize("dtype,n,d,k,iters", [(np.float64, 30_000, 40, 100, 3), (np.float32, 130_001, 64, 260, 3),
-                                               (np.float32, 60_000, 50, 200, 2), (np.float32, 50_000, 64, 100, 5)])
+                                               (np.float32, 60_000, 64, 700, 1), (np.float32, 50_000, 64, 100, 5)])
 def test_values_written_into_an_attached_matrix_are_seen(eng, dtype, n, d, k, iters):
     """Fit, other values into the same device buffer (the same rows in another order, so that max |x| holds), fit and
-    assign without attaching again: what a fresh handle on the new values gives."""
+    assign without attaching again: what a fresh handle on the new values gives.  (Float32 rows of a width that is not a
+    multiple of four are copied once per attachment, as the header says.)"""
     import torch
     rng = np.random.default_rng(d * k)
     centers = rng.uniform(-6, 6, (k, d))
@@ -1750,3 +1751,43 @@ def test_a_refused_matrix_leaves_the_estimator_as_it_was(built_lib, first, secon
             call()
         assert m.double_precision == precision == int(first == np.float64)
         assert np.array_equal(m.cluster_centers_, centers) and np.array_equal(m.predict(X), want)
+
+
+def test_a_single_pass_over_unaligned_rows_takes_no_padded_copy(eng, built_lib):
+    """Labels of a resident matrix whose rows are not 16-byte aligned: with device memory for the rounded rows (124 bytes a
+    row) but not for a padded copy (208), one pass runs.  With centroids that leave every row open the pass is made
+    again on whole rows, for which the rounded ones give way."""
+    import torch
+    from h2o4gpu_b200.libs import lib_kmeans
+    lib = lib_kmeans.cdll()
+    rng = np.random.default_rng(50)
+    n, d, k, mb = 400_000, 50, 64, 1 << 20
+    centers = rng.uniform(-6, 6, (k, d))
+    a = (centers[rng.integers(0, k, n)] + rng.standard_normal((n, d))).astype(np.float32)
+    crowded = (3.0 + 1e-5 * rng.standard_normal((k, d))).astype(np.float32)
+    X = torch.as_tensor(a, device="cuda")
+
+    def assign(C, limit):
+        h = eng.ResidentKMeans()
+        h.attach_device(0, X.data_ptr(), n, d)
+        lib.kmeans_selftest_alloc_limit(limit)
+        try:
+            h.set_centroids(C)
+            h.assign()
+        finally:
+            lib.kmeans_selftest_alloc_limit(-1)
+        out = h.labels(), h.estep_info()
+        h.close()
+        return out
+
+    lab, info = assign(centers, 124 * n + 16 * mb)
+    assert info == (5, False) and _nearest_gap(a, centers.astype(np.float32), lab) == 0
+    lab, info = assign(crowded, 216 * n + 16 * mb)
+    assert info == (5, True) and _nearest_gap(a, crowded, lab) == 0
+    # without memory for a padded copy the kernels that need none take the pass (float32 scores: near ties may differ)
+    lab, info = assign(crowded, 124 * n + 16 * mb)
+    assert info == (5, True)
+    x = a.astype(np.float64)
+    score = (crowded.astype(np.float64) ** 2).sum(1) - 2 * x @ crowded.astype(np.float64).T
+    size = (x * x).sum(1) + (crowded.astype(np.float64) ** 2).sum(1).max()
+    assert (score[np.arange(n), lab] - score.min(1) <= 2 * (d + 2) * 2.0 ** -24 * size).all()
