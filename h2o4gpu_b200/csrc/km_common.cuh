@@ -177,8 +177,8 @@ inline cudaError_t km_free(void* p) {
   return cudaFreeAsync(p, dp.stream[dev]);
 }
 
-// Whether to take `bytes` for a copy that a call can do without (rounded rows): as much again and 1 GB have to stay
-// free, for what this handle and its user allocate later.  Below 256 MB the question costs more than it guards.
+// Whether to take `bytes` for a copy that a call can do without (rounded rows): an eighth of the device has to stay free
+// for what this handle and its user allocate later.  Below 256 MB the question costs more than it guards.
 inline bool km_room_for(size_t bytes) {
   if (bytes < ((size_t)256 << 20)) return true;
   size_t free_b = 0, total_b = 0;
@@ -194,7 +194,7 @@ inline bool km_room_for(size_t bytes) {
         cudaMemPoolGetAttribute(dp.pool[dev], cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess && held > used)
       free_b += held - used;
   }
-  return free_b >= 2 * bytes + ((size_t)1 << 30);
+  return free_b >= bytes + total_b / 8;
 }
 
 inline void km_trim_pools() {
