@@ -1351,8 +1351,9 @@ int Engine<T>::launch_accumulate(Shard<T>& s, T scale, long long* dst, const uns
   return KM_OK;
 }
 
-// The tcgen05 kernel serves float32 shards with d in {32, 64} and 16 < k <= 128 on
-// compute capability 10.x; everything else runs on the SIMT kernels.
+// Whether a tensor-core kernel (tc_kind) labels the shards: checked data on compute capability 10.x, magnitudes the
+// operand scales reach, rows that TMA can address or memory for a copy that it can.  The others run on the SIMT kernels
+// or, in float64, on the matrix unit.
 template <typename T>
 bool Engine<T>::tc_ok(int flags, bool single) const {
   if (flags & KM_FIT_FORCE_SIMT) return false;
@@ -1549,6 +1550,7 @@ int Engine<T>::launch_assign(Shard<T>& s, bool use_tc, bool count_changes) {
       KM_TRY(tc::launch(s.tcp, s.labels, s.st, count_changes, s.amb_rows, s.amb_seg, tc::tol_rel_of(d), s.num_sms,
                         s.stream, bits, s.amb_near, tc_split_build, &launches));
       s.moved_bits_valid = bits != nullptr;
+      if (d == 64 && s.tcp.xsplit_of == s.X) s.estep_kernel = 6;   // on the rounded rows
       const size_t tiles = (s.rows + tc::kBM - 1) / tc::kBM;
       const int n_seg = (int)std::min<size_t>(tiles, (size_t)s.num_sms);
       auto refine = [&](auto fn) {

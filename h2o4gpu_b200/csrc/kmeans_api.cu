@@ -401,7 +401,7 @@ static int estep_info(km::Engine<T>* e, int local, int* kernel, int* whole_rows)
   KM_CUDA(cudaMemcpyAsync(&w, &s.st->full_rows, sizeof(w), cudaMemcpyDeviceToHost, s.stream));
   KM_CUDA(cudaStreamSynchronize(s.stream));
   *kernel = s.estep_kernel;
-  *whole_rows = w != 0;
+  *whole_rows = w != 0 && (s.estep_kernel == 5 || s.estep_kernel == 6);
   return KM_OK;
 }
 

@@ -44,8 +44,9 @@ int kmeans_last_fit_info(int* iterations, double* inertia);
 /* Device buffers come from one memory pool per device that keeps freed memory for the next
  * call (the reference allocates and frees per call through thrust::device_vector,
  * src/gpu/kmeans/kmeans_h2o4gpu.cu:672-683, 795-812).  This returns everything the pools hold
- * and no live handle uses to the driver.  H2O4GPU_KM_POOL=0 in the environment turns the
- * pools off. */
+ * and no live handle uses to the driver, and with it the pinned staging buffers and the worker
+ * streams that copies from and to pageable memory keep (unless such a copy is running).
+ * H2O4GPU_KM_POOL=0 in the environment turns the pools off. */
 int kmeans_trim_memory(void);
 
 /* Every wait inside a kernel (for a peer GPU's flag in the multi-GPU exchanges, for an mbarrier in the
@@ -236,8 +237,8 @@ typedef struct kmeans_stats {
 int kmeans_get_stats(kmeans_handle_t h, kmeans_stats* out);
 /* Which kernel the last label pass over shard `local` ran (of a fit, or kmeans_assign_resident): 0 a SIMT
  * kernel or the float64 matrix unit, 1 small table, 2 streamed table with three products per pair, 3 few centroids
- * and wide rows, 4 both operands streamed, 5 one product per pair on rounded rows.  *whole_rows: 1 when rounded
- * rows (kernels 1 and 5) left too many rows open and the device sent the pass on to the kernel that reads whole
+ * and wide rows, 4 both operands streamed, 5 one product per pair on rounded rows, 6 small table with two products
+ * on rounded rows (64 columns).  *whole_rows: 1 when rounded rows (kernels 5 and 6) left too many rows open and the device sent the pass on to the kernel that reads whole
  * rows.  For tests and for a look at what a data set does. */
 int kmeans_estep_info(kmeans_handle_t h, int local, int* kernel, int* whole_rows);
 /* Sum of squared distances of every row to its assigned centre (direct

@@ -920,7 +920,7 @@ def test_f64_matrix_unit_kernel_matches_simt_kernel_and_oracle(eng, tmp_path):
 
 
 def test_presplit_tensor_core_kernel_matches_converting_kernel(eng, tmp_path):
-    """d = 64, 16 iterations or more: the E-step that reads rows split once into fp16 halves against the kernel that
+    """d = 64, three iterations or more (16 here): the E-step that reads rows rounded once to fp16 against the kernel that
     converts every tile (environment switch, child process): the same labels and centroids, bit for bit;
     and new data at the same address and shape on one handle is not mistaken for the old."""
     import os
@@ -1355,8 +1355,9 @@ def test_random_shapes_one_step_matches_oracle(eng, n, d, k):
 
 # ---- one fp16 product per (row, centroid) with a proven bound, exact pass over the open rows ----
 def _nearest_gap(X, C, labels):
-    """Largest excess of a row's labelled squared distance over its smallest one, and the rows whose label is not the
-    lowest index among exactly equal smallest distances; direct differences in float64 for the few that differ."""
+    """Number of rows whose label is not their nearest centroid, the lowest index of those.  The expanded form in float64
+    finds the rows to look at; direct differences in float64 decide on them, so exact ties count only where that
+    form disagrees with the label (tables with equal centroids have a check of their own)."""
     C = C.astype(np.float64)
     cn = (C * C).sum(1)
     wrong = 0
@@ -1398,9 +1399,16 @@ def test_one_product_kernel_labels_are_the_float64_argmin(eng, dtype, n, d, k, d
     h.upload(X)
     h.fit(C, 0)
     assert h.stats()["path"] == 3
+    # a single pass over few float64 products stays on the matrix unit
+    unit = dtype == np.float64 and d % 2 == 0 and k > 32 and n * k * d < 5e8
+    assert h.estep_info() == ((0, False) if unit else (5, data != "clusters"))
     assert _nearest_gap(X, C, h.labels()) == 0
-    if data != "equal":
+    if data == "equal":     # the lowest index of every group of equal centroids, and no other
+        assert np.isin(h.labels(), np.unique(C, axis=0, return_index=True)[1]).all()
+    else:
         h.fit(C, 3)
+        kernel, whole = h.estep_info()
+        assert kernel == 5 and (whole or data == "clusters")
         got = h.centroids(), h.labels()
         assert _nearest_gap(X, got[0], got[1]) == 0
         h.fit(C, 3, flags=eng.FIT_FULL_SUMS)
@@ -1791,3 +1799,28 @@ def test_a_single_pass_over_unaligned_rows_takes_no_padded_copy(eng, built_lib):
     score = (crowded.astype(np.float64) ** 2).sum(1) - 2 * x @ crowded.astype(np.float64).T
     size = (x * x).sum(1) + (crowded.astype(np.float64) ** 2).sum(1).max()
     assert (score[np.arange(n), lab] - score.min(1) <= 2 * (d + 2) * 2.0 ** -24 * size).all()
+
+
+@pytest.mark.parametrize("n,k,iters", [(20_000, 100, 3), (20_000, 17, 5), (6001, 128, 4), (127, 33, 3)])
+@pytest.mark.parametrize("data", ["clusters", "close"])
+def test_rounded_rows_of_the_small_table_give_way_when_they_leave_rows_open(eng, n, k, iters, data):
+    """64 columns, up to 128 centroids: rows and centroids so close together that the bound of the rounded rows leaves more
+    than a quarter of them open send the E-steps on to the kernel that converts whole rows; separated ones do not.
+    Labels are the float64 argmin either way, and incremental and full sums agree bit for bit."""
+    rng = np.random.default_rng(n + k)
+    if data == "close":
+        X = (3.0 + 1e-3 * rng.standard_normal((n, 64))).astype(np.float32)
+    else:
+        X = (rng.uniform(-6, 6, (k, 64))[rng.integers(0, k, n)] + rng.standard_normal((n, 64))).astype(np.float32)
+    C = X[rng.choice(n, k, replace=False)].copy()
+    h = eng.ResidentKMeans()
+    h.upload(X)
+    h.fit(C, iters)
+    assert h.estep_info() == (6, data == "close")
+    refined = h.stats()["refined_rows"]
+    assert refined == iters * n if data == "close" else refined < iters * n // 4
+    got = h.centroids(), h.labels()
+    assert _nearest_gap(X, got[0], got[1]) == 0
+    h.fit(C, iters, flags=eng.FIT_FULL_SUMS)
+    assert np.array_equal(got[0], h.centroids()) and np.array_equal(got[1], h.labels())
+    h.close()
