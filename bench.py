@@ -226,7 +226,9 @@ def run_case(ctx, w, K, W, flags, dtype=np.float32, weighted=False, min_seconds=
     h.attach_device(0, X.data_ptr(), n, d, n_total=n * ctx.world)
     if weighted:
         h.set_sample_weight(np.random.default_rng(11 + ctx.rank).gamma(2.0, 1.5, n).astype(dtype))
-    # per-upload preparation (row norms, fp16-split copy of the rows for the d = 64 kernel) happens in the warm-up
+    # what is prepared once per attachment (row norms, the rounded rows of the d = 64 kernel) happens in the warm-up;
+    # the rounded rows of larger tables are made by every fit ahead of its loop: in the wall and end-to-end times, not in
+    # the device time of the loop
     if W > 0:
         h.fit(init, W, flags=flags)
     sampler = ClockSampler(ctx.local_rank) if (sample_clocks and ctx.rank == 0) else None
@@ -263,7 +265,7 @@ def run_case(ctx, w, K, W, flags, dtype=np.float32, weighted=False, min_seconds=
            "wall_ms_per_step": 1e3 * med["_wall"] / steps,
            "value": ctx.world * n * steps / (med["_dev_ms"] * 1e-3),
            "ms_loop_per_rank": ctx.gather(med["ms_loop"] + med["ms_final_assign"]),
-           "stats": med, "clocks": clocks, "timed_seconds": wall_all, "init": init}
+           "stats": med, "estep": h.estep_info(), "clocks": clocks, "timed_seconds": wall_all, "init": init}
     out["idle_ms_per_step"] = out["ms_per_step"] - out["assign_ms"] - out["update_ms"] - med["ms_final_assign"] / steps
     if after_fit is not None:
         out["after"] = after_fit(h, X)
@@ -275,7 +277,13 @@ def roofline_of(args_workload, r, hbm_peak, tensor_peak, peak_kind):
     """Roofline object of the dominant kernel of a finished case."""
     n, d, k = r["n"], r["d"], r["k"]
     st = r["stats"]
-    alg_bytes = n * (d * 4 + 4)
+    kernel, whole = r["estep"]
+    rounded = kernel in (5, 6) and not whole
+    # what a launch has to move per row: the float32 row and a label, or the row rounded to fp16, the two floats its
+    # error bound needs, and a label
+    alg_bytes = n * (d * 2 + 8 + 4 if rounded else d * 4 + 4)
+    # half-precision products per (row, centroid): one or two on rounded rows, three for float32 accuracy
+    products = {5: 1, 6: 2}[kernel] if rounded else 3
     a_ms, u_ms = r["assign_ms"], r["update_ms"]
     # the dominant kernel is the one that streams X every iteration: distance + argmin (with the fused
     # small-k kernel it also forms the sums); the M-step moves only the rows whose label changed
@@ -284,25 +292,26 @@ def roofline_of(args_workload, r, hbm_peak, tensor_peak, peak_kind):
     flops = 2.0 * n * k * d
     # DRAM bytes per row of the dominant kernel from the committed ncu captures (profiles/), taken on
     # a smaller case of the same shape and scaled by the rows of a launch (traffic grows in proportion)
-    ncu_bytes_per_row = {("c2", 3): 269.2, ("c3", 3): 527.7, ("c4", 3): 3163.3, ("c5", 3): 1063.4,
-                         ("c4_k100", 3): 3162.5}.get((args_workload, st["path"]))
+    ncu_bytes_per_row = {("c2", 6): 144.9, ("c3", 5): 276.0, ("c4", 3): 3163.3, ("c5", 5): 544.6,
+                         ("c4_k100", 4): 3162.5}.get((args_workload, kernel)) if not whole else None
     traffic = ncu_bytes_per_row * n if ncu_bytes_per_row else None
-    tens = {"fp32_equiv_tflops": flops / (a_ms * 1e-3) / 1e12, "issued_tflops": 3 * flops / (a_ms * 1e-3) / 1e12,
-            "peak_tflops": tensor_peak, "frac": 3 * flops / (a_ms * 1e-3) / 1e12 / tensor_peak}
+    issued = products * flops / (a_ms * 1e-3) / 1e12
+    tens = {"fp32_equiv_tflops": flops / (a_ms * 1e-3) / 1e12, "issued_tflops": issued, "products_per_pair": products,
+            "peak_tflops": tensor_peak, "frac": issued / tensor_peak}
     hbm = {"bound": "hbm", "achieved": achieved, "peak": hbm_peak, "unit": "GB/s", "frac": achieved / hbm_peak,
            "traffic": traffic, "peak_kind": "of " + peak_kind,
            "kernel": "distance+argmin" if st["path"] != 1 else "distance+argmin+sums (fused)",
            "algorithmic_bytes_per_launch": alg_bytes,
            "whole_step_frac": alg_bytes / (r["ms_per_step"] * 1e-3) / 1e9 / hbm_peak}
-    if st["path"] == 3 and tens["frac"] > hbm["frac"]:
-        # large centroid tables: the distance kernel is bound by the tensor pipe (2kd flops per row, three
-        # half-precision products per flop pair); peak = measured bf16 GEMM burst
+    if kernel and tens["frac"] > hbm["frac"]:
+        # large centroid tables: the distance kernel is bound by the tensor pipe (2kd flops per row and product);
+        # peak = measured bf16 GEMM burst
         roof = {"bound": "tensor", "achieved": tens["issued_tflops"], "peak": tens["peak_tflops"],
                 "unit": "TFLOP/s", "frac": tens["frac"], "traffic": traffic, "peak_kind": "of " + peak_kind,
-                "kernel": "distance+argmin", "algorithmic_flops_per_launch": 3 * flops, "hbm_frac": hbm["frac"]}
+                "kernel": "distance+argmin", "algorithmic_flops_per_launch": products * flops, "hbm_frac": hbm["frac"]}
     else:
         roof = hbm
-    return roof, (tens if st["path"] == 3 else None)
+    return roof, (tens if kernel else None)
 
 
 def brief(r, roof):
