@@ -1,5 +1,5 @@
-// Tensor-core distance + argmin in one fp16 product per (row, centroid), with a proven error bound and an exact
-// pass over the rows the bound leaves open: float32 and float64 rows of up to 256 columns, more than 16 centroids.
+// Tensor-core distance + argmin in one fp16 product per (row, centroid), with an error bound and an exact pass
+// over the rows the bound leaves open: float32 and float64 rows of up to 256 columns, more than 16 centroids.
 //
 // Replaces calculate_distances + relabel (src/gpu/kmeans/kmeans_labels.cu:115-244, kmeans_labels.h:360-392).
 //
@@ -7,7 +7,8 @@
 // float64 rows went to the float64 matrix unit, which is forty times slower than this one.  A label does not need
 // that: the rows are rounded once to fp16 (half_rows_kernel: two bytes per element and, per row, |x|^2 and the
 // length of what the rounding dropped), the scores |c|^2 - 2 x.c are formed from the rounded operands, and the
-// lengths of the dropped parts bound how far the difference of two scores can be off (half_tolerance).  A row
+// lengths of the dropped parts bound how far the difference of two scores can be off (half_tolerance: that part is
+// Cauchy-Schwarz; the tensor core's own accumulation enters with the measured constant of tol_rel_of).  A row
 // whose best score is ahead of every other by more than that has its label; the others are listed with the few
 // centroids that can still be nearest and settled in double precision from the unrounded rows
 // (half_exact_f32_kernel, half_exact_f64_kernel).  Labels are therefore those of exact arithmetic, as before.
@@ -139,7 +140,7 @@ half_rows_kernel(const T* __restrict__ X, size_t n, int d, int ldh, int lpr, flo
   }
 }
 
-// Bound by the tensor pipe at 256 columns (1.33 - 1.48 PFLOP/s; a library GEMM reaches 1.6), below that by the
+// Bound by the tensor pipe at 256 columns (92 % of its cycles; 1.54 PFLOP/s, a library GEMM 1.69), below that by the
 // hand-over of the accumulator between the MMAs and the epilogue (128 columns: 1.0, 64: 0.56 PFLOP/s).  2e6 x 128 rows
 // with 1000 centroids: 0.48 ms per pass (three-term kernel 1.20), 5e5 x 256 with 4096: 0.68 (2.12), 60,000 x 256
 // float64 rows with 4096: 0.10 (float64 matrix unit 5.7).  What made the three-term kernel's layout unfit:

@@ -359,8 +359,10 @@ __device__ __forceinline__ void block_argmax(double& bv, unsigned long long& br,
 // threads.  Non-negative doubles order as their bits, so 11 bits at a time from the top: count the values by those
 // bits among the ones that agree with the choice so far, and choose the bits that hold the E-th.  Ends early when
 // so few values reach the choice that more bits would not shorten the list of candidates.  0 if there are fewer than E.
-// hist: 2048 words of shared memory.  Bound by the reads from L2 (m / 256 per thread and round); 37,888 values, two
-// to three rounds.
+// hist: 2048 words of shared memory.  Bound by the reads from L2 (m / 256 per thread and round).  M-step of 1e6 x 8
+// rows with 53 / 250 / 1000 empty clusters: 0.18 / 0.21 / 0.54 ms; with the maxima of warps, or one maximum per round
+// where those are too few: 0.18 / 0.21 / 16.5, and 0.56 / 2.0 / 16.9 when 40,000 far rows lie together (here 0.15 /
+// 0.19 / 0.88).
 __device__ double kth_largest(const double* v, int m, int E, unsigned int* hist) {
   __shared__ unsigned int s_wsum[8], s_bin, s_above, s_count;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -527,8 +529,8 @@ relocate_kernel(const T* __restrict__ X, size_t n, int d, const int* __restrict_
   if (E > kFarDirectMax && top_far(grid, dist, n, E, fs, s_v, s_r, s_i, &n_far)) {
     // the farthest rows are known and ordered, the e-th goes to the e-th empty cluster.  A CTA per row, all rows out
     // of their donors first: two may share a donor, but the sums are integers and no row's move depends on another's.
-    // (One CTA moving them in turn, and finding them one maximum per round, took 20 us for each: 53 rows 1.07 ms, now
-    // 0.12 ms with the search.)
+    // (One CTA moving them in turn, and finding them one maximum per round, took 20 us for each: 53 rows of 1e6 x 8
+    // 1.07 ms, now 0.13 ms with the search.)
     grid.sync();
     if (!(__ldcg(fs.oval) > 0.0)) return;
     for (int phase = 0; phase < 2; ++phase) {

@@ -16,7 +16,7 @@
 namespace km {
 
 constexpr int kNarrowThreads = 256;
-constexpr int kNarrowPiece = 1024;    // centroids in shared memory at a time (at most 96 KB)
+constexpr int kNarrowPiece = 1024;    // centroids in shared memory at a time (at most 80 KB)
 constexpr int kNarrowMaxD = 8;
 
 // doubles / floats per centroid in shared memory: a whole number of 16-byte vectors
