@@ -308,17 +308,15 @@ struct Engine : EngineBase {
     if (lent() && (std::is_same<T, double>::value || d % 4 == 0))
       for (auto& s : shards) s.tchp.of = nullptr;
   }
-  // Whether rounding the rows pays for `passes` label passes.  Float32 rows of a lent matrix: rounding takes about 1.6 ps
-  // per element, the one-product kernel saves 2.5 fs per element and centroid (500,000 x 128 and 1e6 x 64 rows).
-  // Float64 rows in a single pass: the float64 matrix unit takes 0.069 ps per product, 5e8 of them what the four
-  // further launches and the rounding do (60,000 x 40, 50 centroids: 101 us a call against 118; 200,000 x 64, 100
-  // centroids: 240 against 170); without the unit (odd widths) the FP64 pipe is behind earlier.
-  bool rounding_pays(int passes) const {
-    if (std::is_same<T, float>::value) return d % 4 != 0 || !lent() || (double)passes * k >= 640.0;
-    if (passes > 1 || d % 2 != 0 || k <= 32) return true;
-    size_t rows = 0;
-    for (const auto& s : shards) rows = std::max(rows, s.rows);
-    return (double)rows * k * d >= 5e8;
+  // Whether rounding the rows of a lent matrix pays for `passes` label passes.  Float32: rounding takes about 1.6 ps per
+  // element, the one-product kernel saves 2.5 fs per element and centroid (500,000 x 128 and 1e6 x 64 rows).  Float64 rows
+  // in a single pass: the float64 matrix unit takes 0.069 ps per product, 5e8 of them what the four further launches
+  // and the rounding do (60,000 x 40, 50 centroids: 101 us a call against 118; 200,000 x 64, 100 centroids: 240 against
+  // 170); without the unit (odd widths, few centroids) the FP64 pipe is behind earlier.
+  bool rounding_pays(const Shard<T>& s, int passes) const {
+    if (!lent()) return true;   // once per upload
+    if (std::is_same<T, float>::value) return d % 4 != 0 || (double)passes * k >= 640.0;
+    return passes > 1 || !dmma::shape_ok(k, d) || (double)s.rows * k * d >= 5e8;
   }
   int fit_passes = 1;   // label passes of the running fit
   double xmax_all() const {
@@ -1384,7 +1382,7 @@ template <typename T>
 int Engine<T>::tc_refresh(Shard<T>& s, Pass pass, bool for_labels) {
   const OutRule rule = for_labels ? out_rule(xmax_all(), d) : OutRule{};
   const bool half = pass != Pass::whole && half_shape_ok() && (tc_kind() == 2 || tc_kind() == 5) &&
-                    rounding_pays(pass == Pass::fit ? fit_passes : 1);
+                    rounding_pays(s, pass == Pass::fit ? fit_passes : 1);
   s.tchp.on = s.tchp.alone = false;
   if constexpr (std::is_same<T, double>::value) {
     double xmax = 0;

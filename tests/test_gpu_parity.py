@@ -1399,9 +1399,7 @@ def test_one_product_kernel_labels_are_the_float64_argmin(eng, dtype, n, d, k, d
     h.upload(X)
     h.fit(C, 0)
     assert h.stats()["path"] == 3
-    # a single pass over few float64 products stays on the matrix unit
-    unit = dtype == np.float64 and d % 2 == 0 and k > 32 and n * k * d < 5e8
-    assert h.estep_info() == ((0, False) if unit else (5, data != "clusters"))
+    assert h.estep_info() == (5, data != "clusters")
     assert _nearest_gap(X, C, h.labels()) == 0
     if data == "equal":     # the lowest index of every group of equal centroids, and no other
         assert np.isin(h.labels(), np.unique(C, axis=0, return_index=True)[1]).all()
@@ -1824,3 +1822,34 @@ def test_rounded_rows_of_the_small_table_give_way_when_they_leave_rows_open(eng,
     h.fit(C, iters, flags=eng.FIT_FULL_SUMS)
     assert np.array_equal(got[0], h.centroids()) and np.array_equal(got[1], h.labels())
     h.close()
+
+
+@pytest.mark.parametrize("dtype,n,d,k,iters,kernel", [
+    (np.float32, 55_000, 64, 600, 0, 2), (np.float32, 55_000, 64, 600, 1, 5), (np.float32, 60_000, 64, 640, 0, 5),
+    (np.float32, 110_000, 64, 300, 1, 2), (np.float32, 110_000, 64, 300, 2, 5), (np.float32, 50_000, 50, 300, 0, 5), (np.float64, 20_000, 40, 200, 0, 0),
+    (np.float64, 20_000, 40, 200, 1, 5), (np.float64, 20_000, 40, 700, 0, 5), (np.float64, 20_000, 41, 200, 0, 5)])
+def test_rows_of_a_lent_matrix_are_rounded_where_that_pays(eng, dtype, n, d, k, iters, kernel):
+    """Single passes and short fits on both sides of the limits (2e9 products, 640 centroids x passes, 5e8 float64
+    products): the kernel that runs, and labels equal to those of an uploaded matrix, whose rows are rounded once."""
+    import torch
+    rng = np.random.default_rng(n + k)
+    centers = rng.uniform(-6, 6, (k, d))
+    a = (centers[rng.integers(0, k, n)] + rng.standard_normal((n, d))).astype(dtype)
+    C = a[rng.choice(n, k, replace=False)].copy()
+    X = torch.as_tensor(a, device="cuda")
+    h, up = eng.ResidentKMeans(dtype=dtype), eng.ResidentKMeans(dtype=dtype)
+    h.attach_device(0, X.data_ptr(), n, d)
+    up.upload(a)
+    if iters:
+        h.fit(C, iters)
+        up.fit(C, iters)
+    else:
+        for e in (up, h):
+            e.set_centroids(C)
+            e.assign()
+    assert h.estep_info() == (kernel, False)
+    lab = h.labels()
+    assert np.array_equal(lab, up.labels()) and np.array_equal(h.centroids(), up.centroids())
+    assert _nearest_gap(a, h.centroids(), lab) == 0
+    h.close()
+    up.close()
