@@ -4,10 +4,11 @@
 // The tile kernel pads a row to 16 columns: with three columns four fifths of its arithmetic are on zeros.  Here a
 // thread keeps R rows in registers and walks the centroids, which all lanes read together from shared memory
 // (d coordinates and |c|^2, padded to a vector load); the table passes through shared memory in pieces if it is
-// large.  Bound by the FP64 pipe for float64 (d + 2 instructions per score), by issue for float32.  273,280 x 3
-// float64 rows, 64 centroids: 117 us with the tile kernel, 18 us now.  The arithmetic is the tile kernel's - a chain
-// of fused multiply-adds over the columns, then |c|^2 - 2 x.c, first minimum wins - so the labels are the same bit
-// for bit.
+// large.  273,280 x 3 float64 rows, 64 centroids: 117 us with the tile kernel, 18 us now.  2e7 rows of them take
+// 1.05 ms: the FP64 pipe at a third of its rate (d + 2 instructions per score) and issue slots half busy, the
+// rest waits for the rows, which a thread loads before its first score.  The arithmetic is the tile kernel's - a
+// chain of fused multiply-adds over the columns, then |c|^2 - 2 x.c, first minimum wins - so the labels are the
+// same bit for bit.
 #pragma once
 
 #include "km_common.cuh"
