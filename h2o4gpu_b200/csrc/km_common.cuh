@@ -366,9 +366,9 @@ __device__ bool left_out(const OutRule& rule, const T* __restrict__ c, int d, co
   float l1 = 0.f;
   for (int t = 0; t < d; ++t) l1 += fabsf((float)c[t]);
   if (!rule((float)cnorm[j], l1)) return false;
-  for (int i = 0; i < k; ++i)
-    if ((float)cnorm[i] <= rule.rr) return true;
-  return false;
+  bool within = false;
+  for (int i = threadIdx.x; i < k; i += blockDim.x) within = within || (float)cnorm[i] <= rule.rr;
+  return __syncthreads_or(within);
 }
 
 template <typename T> struct Inf;

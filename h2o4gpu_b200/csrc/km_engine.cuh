@@ -303,7 +303,11 @@ struct Engine : EngineBase {
   // anew in every pass are therefore rounded anew by every call; what was always taken once per attachment stays (max
   // |x|, row norms, the copies of rows that are not 16-byte aligned and of long fits at 64 columns).  A matrix this
   // handle uploaded cannot change under it.
-  bool lent() const { return !shards.empty() && shards[0].X != shards[0].X_owned; }
+  bool lent() const {
+    for (const auto& s : shards)
+      if (s.X != s.X_owned) return true;
+    return false;
+  }
   void drop_row_copies() {
     if (lent() && (std::is_same<T, double>::value || d % 4 == 0))
       for (auto& s : shards) s.tchp.of = nullptr;
