@@ -259,6 +259,8 @@ int Engine<T>::fit(int k_, int max_iter, double threshold, const T* init, int fl
       KM_CUDA(cudaMemsetAsync(s.pflush, 0, s.gacc_count(k, d) * kFlushPad * sizeof(long long), s.stream));
     if (use_tc) KM_TRY(tc_refresh(s, Pass::fit));
   }
+  // (float64 rows that could not be rounded, or do not pay for it, stay on the matrix unit or the SIMT kernels)
+  if (use_tc && std::is_same<T, double>::value && !shards[0].tchp.on) stats.path = 2;
 
   // events on shard 0: [4*it + 0..3] = start, after E-step, after sums, after close
   Shard<T>& s0 = shards[0];

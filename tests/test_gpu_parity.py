@@ -1586,6 +1586,7 @@ def test_a_fit_that_fits_without_the_rounded_rows_runs(eng, built_lib, dtype, d,
         finally:
             lib.kmeans_selftest_alloc_limit(-1)
         out = h.centroids(), h.labels()
+        assert h.stats()["path"] == (3 if h.estep_info()[0] else 2)
         h.close()
         return out
 
